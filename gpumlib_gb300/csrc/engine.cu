@@ -21,6 +21,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -138,6 +139,11 @@ struct Sizes {
 
 static Sizes compute_sizes(int rule, int n, int m, int r, int precision) {
     Sizes z{};
+    if (precision == GPUNMF_FP32 && sp_supported(n, m, r)) {  // products on the tensor cores: no FP32 workspaces
+        z.s_h = z.s_w = z.s_g = 1;
+        z.red = std::max(2 * (size_t)wh_reduce_ctas(n, m), (size_t)quality_ew_ctas((long long)n * m));
+        return z;
+    }
     z.s_h = gemm_f32_splits(r, m, n);
     z.s_w = gemm_f32_splits(n, r, m);
     int sg1 = gemm_f32_splits(r, r, n), sg2 = gemm_f32_splits(r, r, m);
@@ -162,6 +168,7 @@ size_t job_footprint(int rule, int n, int m, int r, int precision) {
                     z.wh + (size_t)r * r + (size_t)r + 8;
     size_t bytes = floats * sizeof(float) + z.red * sizeof(double) + 64;
     if (precision == GPUNMF_BF16) bytes += tc_footprint(rule, n, m, r);
+    if (sp_supported(n, m, r)) bytes += sp_footprint(rule, n, m, r, precision == GPUNMF_BF16);
     return bytes;
 }
 
@@ -171,6 +178,7 @@ size_t job_footprint(int rule, int n, int m, int r, int precision) {
 static void job_free(gpunmf_job *j) {
     if (!j) return;
     if (j->tc) tc_destroy(j);
+    sp_destroy(j);
     float *fl[] = {j->V, j->W, j->H, j->P_h, j->P_w, j->P_g, j->G, j->D_h, j->D_w, j->WH, j->sums, j->d_quality};
     for (float *p : fl) job_dev_free(j, p);
     job_dev_free(j, j->red);
@@ -277,6 +285,7 @@ static gpunmf_status job_alloc(int rule, int n, int m, int r, float eps, int pre
         }
     }
     if (st == GPUNMF_OK && precision == GPUNMF_BF16) st = tc_create(j);
+    if (st == GPUNMF_OK && precision == GPUNMF_FP32 && sp_supported(n, m, r)) st = sp_create(j, false);
     if (st != GPUNMF_OK) {
         job_free(j);
         return st;
@@ -314,6 +323,7 @@ static gpunmf_status job_upload(gpunmf_job *j, const float *V, const float *W, c
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(j->W, W, nr * sizeof(float), kind, j->stream));
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(j->H, H, rm * sizeof(float), kind, j->stream));
     if (j->precision == GPUNMF_BF16) TRY_STATUS(tc_prepare(j, v_src));
+    if (j->sp) TRY_STATUS(sp_prepare(j, false));
     return GPUNMF_OK;
 }
 
@@ -361,7 +371,16 @@ static gpunmf_status quality_step(gpunmf_job *j, bool fused_wh) {
         GPUNMF_CUDA_TRY(cudaEventRecord(j->qev, s));
         j->q_pending = true;
         return GPUNMF_OK;
-    } else if (fused_wh) {
+    }
+    if (j->precision == GPUNMF_FP32 && j->sp) {  // one launch, which writes the read-back word too
+        TRY_STATUS(sp_quality(j));
+        if (!sp_quality_writes_host(j))
+            GPUNMF_CUDA_TRY(cudaMemcpyAsync(j->h_quality(), j->d_quality, sizeof(float), cudaMemcpyDeviceToHost, s));
+        GPUNMF_CUDA_TRY(cudaEventRecord(j->qev, s));
+        j->q_pending = true;
+        return GPUNMF_OK;
+    }
+    if (fused_wh) {
         GPUNMF_CUDA_TRY(wh_quality_f32(n, m, r, j->W, j->H, j->V, j->eps, j->red, s));
         GPUNMF_CUDA_TRY(finalize_partials(j->red, wh_reduce_ctas(n, m), 1, 0, j->d_quality, nullptr, s));
     } else {
@@ -466,6 +485,8 @@ static gpunmf_status job_iterate(gpunmf_job *j, int iters, bool updateW) {
         gpunmf_status st;
         if (j->precision == GPUNMF_BF16)
             st = tc_iterate(j, updateW);
+        else if (j->sp)
+            st = sp_iterate(j, updateW);
         else if (rule_is_kl(j->rule))
             st = iterate_kl_f32(j, updateW);
         else
@@ -489,8 +510,29 @@ gpunmf_status job_create_empty(int rule, int n, int m, int r, float eps, int pre
     return job_alloc(rule, n, m, r, eps, precision, (void *)stream, out, pinned64, async_alloc, cta_cap);
 }
 
+// V elements from which the residual runs on the tensor cores: a call on a 64 x 64 job takes 28 us by the
+// FP32 kernel and 35 us there (BF16 job: 40 and 46), on 256 x 256 51 and 35 (62 and 45), on 4096 x 4096
+// 248 and 61 (259 and 73).
+constexpr long long kSplitResidualMin = 32768;
+static bool split_residual(const gpunmf_job *j) { return (long long)j->n * j->m >= kSplitResidualMin; }
+
 gpunmf_status job_prepare(gpunmf_job *j) {
-    if (j->precision == GPUNMF_BF16) return tc_prepare(j);
+    if (j->precision == GPUNMF_BF16) TRY_STATUS(tc_prepare(j));
+    if (j->sp) TRY_STATUS(sp_prepare(j, false));
+    return GPUNMF_OK;
+}
+
+// Before a job's first residual: a BF16 job gets what the tensor-core residual needs, where that is the
+// faster one.  Without the memory for it the FP32 kernel serves.
+void job_residual_ready(gpunmf_job *j) {
+    if (j->sp || j->precision != GPUNMF_BF16 || !sp_supported(j->n, j->m, j->r) || !split_residual(j)) return;
+    if (sp_create(j, true) != GPUNMF_OK || sp_prepare(j, true) != GPUNMF_OK) sp_destroy(j);
+}
+
+gpunmf_status job_residual(gpunmf_job *j, double *d_out) {
+    if (j->sp && split_residual(j)) return sp_residual(j, d_out);
+    GPUNMF_CUDA_TRY(wh_residual_f32(j->n, j->m, j->r, j->W, j->H, j->V, j->red, j->stream));
+    GPUNMF_CUDA_TRY(finalize_partials(j->red, wh_reduce_ctas(j->n, j->m), 2, 1, nullptr, d_out, j->stream));
     return GPUNMF_OK;
 }
 
@@ -687,8 +729,8 @@ gpunmf_status gpunmf_residual_fp64(gpunmf_handle h, double *out) {
     CHECK_HANDLE(h);
     if (!out) return GPUNMF_ERR_INVALID;
     cudaStream_t s = h->stream;
-    GPUNMF_CUDA_TRY(wh_residual_f32(h->n, h->m, h->r, h->W, h->H, h->V, h->red, s));
-    GPUNMF_CUDA_TRY(finalize_partials(h->red, wh_reduce_ctas(h->n, h->m), 2, 1, nullptr, h->d_scalar, s));
+    job_residual_ready(h);
+    TRY_STATUS(job_residual(h, h->d_scalar));
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(h->h_scalar(), h->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, s));
     GPUNMF_CUDA_TRY(cudaStreamSynchronize(s));
     *out = h->h_scalar()[0];

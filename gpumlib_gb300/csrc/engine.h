@@ -8,6 +8,7 @@
 #include "../../include/gpunmf.h"
 
 struct TcState;  // tensor-core path state (tc_kernels.cu)
+struct SpState;  // FP32 products on the tensor cores (split_f32.cuh)
 
 struct gpunmf_job {
     int rule = 0, n = 0, m = 0, r = 0, precision = 0;
@@ -49,6 +50,7 @@ struct gpunmf_job {
     std::vector<cudaEvent_t> tev;
 
     TcState *tc = nullptr;
+    SpState *sp = nullptr;  // FP32 jobs of rank <= 128; BF16 jobs of such ranks for their residual
 
     // allocation mode: jobs made by the server use the stream-ordered allocator on their
     // stream (no device-wide synchronisation on free) and a pinned block owned by the server
@@ -103,4 +105,19 @@ void tc_set_wait_limit(gpunmf_job *j, long long cycles);  // <= 0: the default (
 gpunmf_status tc_inject_missing_arrival(gpunmf_job *j);
 void tc_set_grid_limit(int ctas);         // CTAs per launch of jobs created later (0: one per SM)
 void tc_destroy(gpunmf_job *j);
+
+// FP32 products on the tensor cores (split_f32.cuh): all of an FP32 job's iteration and sampling, or
+// (residual_only) a BF16 job's residual
+bool sp_supported(int n, int m, int r);
+size_t sp_footprint(int rule, int n, int m, int r, bool residual_only);
+gpunmf_status sp_create(gpunmf_job *j, bool residual_only);
+gpunmf_status sp_prepare(gpunmf_job *j, bool residual_only);  // after V, W, H are on the device
+gpunmf_status sp_iterate(gpunmf_job *j, bool updateW);
+gpunmf_status sp_quality(gpunmf_job *j);
+bool sp_quality_writes_host(const gpunmf_job *j);
+gpunmf_status sp_residual(gpunmf_job *j, double *d_out);
+void sp_destroy(gpunmf_job *j);
+void job_residual_ready(gpunmf_job *j);  // before the first job_residual (may allocate)
+// the job's relative residual, enqueued on its stream, into *d_out
+gpunmf_status job_residual(gpunmf_job *j, double *d_out);
 }  // namespace gpunmf

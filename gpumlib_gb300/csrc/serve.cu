@@ -150,9 +150,8 @@ static gpunmf_status chunk_body(gpunmf_server *S, SJob *q, int chunk) {
     gpunmf_status st = job_run(j, chunk, true);
     if (st != GPUNMF_OK) return st;
     cudaStream_t s = j->stream;
-    const int ctas = wh_reduce_ctas(j->n, j->m);
-    GPUNMF_CUDA_TRY(wh_residual_f32(j->n, j->m, j->r, j->W, j->H, j->V, j->red, s));
-    GPUNMF_CUDA_TRY(finalize_partials(j->red, ctas, 2, 1, nullptr, S->d_res + q->slot, s));
+    st = job_residual(j, S->d_res + q->slot);
+    if (st != GPUNMF_OK) return st;
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(S->h_res + q->slot, S->d_res + q->slot, sizeof(double), cudaMemcpyDeviceToHost, s));
     return GPUNMF_OK;
 }
@@ -208,6 +207,7 @@ static gpunmf_status start_job(gpunmf_server *S, SJob *q) {
     q->job->q_interval = 0;
     st = generate_job_data(q->job, q->seed, S->sigma);
     if (st == GPUNMF_OK) st = job_prepare(q->job);
+    if (st == GPUNMF_OK) job_residual_ready(q->job);
     if (st == GPUNMF_OK && S->max_iters >= S->check_every) st = capture_chunk(S, q);
     if (st == GPUNMF_OK) st = enqueue_chunk(S, q);
     return st;

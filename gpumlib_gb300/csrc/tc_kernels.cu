@@ -1491,6 +1491,29 @@ __global__ void convert_h_kernel(const float *__restrict__ H, int r, int m, __nv
     }
 }
 
+// x = x0 + x1 + x2 exactly, each part the nearest BF16 of what is left, in the top half of a word (the
+// FP32 products on the tensor cores, split_f32.cuh).  An infinity or NaN is its first part alone; a
+// value that would round to infinity is cut by truncation.
+__device__ __forceinline__ void cut3(float x, uint32_t &p0, uint32_t &p1, uint32_t &p2) {
+    const float a = fabsf(x) < 3.3e38f ? __bfloat162float(__float2bfloat16_rn(x))
+                                       : __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
+    const float r1 = fabsf(x) < __int_as_float(0x7F800000) ? x - a : 0.f;
+    const float b = __bfloat162float(__float2bfloat16_rn(r1));
+    p0 = __float_as_uint(x != x ? x : a);
+    p1 = __float_as_uint(b);
+    p2 = __float_as_uint(r1 - b);
+}
+// the top halves of two words, the first one's in the low half
+__device__ __forceinline__ uint32_t pack_top(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x7632); }
+__device__ __forceinline__ void store_cut(__nv_bfloat16 *dst, long long part, float x) {
+    uint32_t p0, p1, p2;
+    cut3(x, p0, p1, p2);
+    unsigned short *d = reinterpret_cast<unsigned short *>(dst);
+    d[0] = (unsigned short)(p0 >> 16);
+    d[part] = (unsigned short)(p1 >> 16);
+    d[2 * part] = (unsigned short)(p2 >> 16);
+}
+
 // ------------------------------------------------------------------------
 // update kernel (FP32): the multiplicative rule of nmf_kernels.cu:43-47 (or the
 // additive rule of nmf_kernels.cu:31-38) on an
@@ -1521,7 +1544,22 @@ struct UpdParams {
     float eps;
     int update;               // 0: only write the Gram partials of X (initialisation)
     int additive;             // 1: X = max(0, X + (X / den) (num - den)) (nmf_kernels.cu:31-38)
+    __nv_bfloat16 *Xs;        // FP32 products: the three parts of X instead of Xb, at part * q + c * RP + a
+    long long part;
+    const float *V, *F;       // FP32 products: V (column-major) and the other factor, for plain_sum
+    int K;
 };
+
+// A numerator of the FP32 products by plain FP32 fused multiply-adds, where the sum of the parts'
+// products is not finite: a part of an infinity or NaN has lost which of the two it was.
+template <bool IS_W>
+__device__ __noinline__ float plain_sum(const UpdParams &p, int row, int a) {
+    float s = 0.f;
+    for (int k = 0; k < p.K; k++)
+        s = IS_W ? fmaf(p.V[(long long)k * p.cols + row], p.F[(long long)k * p.r + a], s)
+                 : fmaf(p.V[(long long)row * p.K + k], p.F[(long long)a * p.K + k], s);
+    return s;
+}
 
 template <int RP, bool IS_W>
 __global__ void __launch_bounds__(kUpdThreads) tc_update_kernel(UpdParams p) {
@@ -1624,6 +1662,8 @@ __global__ void __launch_bounds__(kUpdThreads) tc_update_kernel(UpdParams p) {
 #pragma unroll
         for (int j = 0; j < PER; j++) {
             const int k = tid + j * kUpdThreads, c = k / RP, a = k % RP;
+            if (p.Xs && !(fabsf(acc[j]) < __int_as_float(0x7F800000)) && a < r && c < ncol)
+                acc[j] = plain_sum<IS_W>(p, c0 + c, a);
             Ns[a * LDX + c] = acc[j];
         }
     }
@@ -1689,7 +1729,7 @@ __global__ void __launch_bounds__(kUpdThreads) tc_update_kernel(UpdParams p) {
                 if (a < r && c < ncol) {
                     float x = Xn[c * LDN + a];
                     p.X[(long long)a * p.ldx + c0 + c] = x;
-                    p.Xb[(long long)a * p.ldb + c0 + c] = __float2bfloat16_rn(x);
+                    if (p.Xb) p.Xb[(long long)a * p.ldb + c0 + c] = __float2bfloat16_rn(x);
                 }
             }
         } else {
@@ -1697,11 +1737,17 @@ __global__ void __launch_bounds__(kUpdThreads) tc_update_kernel(UpdParams p) {
                 int c = k / RP, a = k % RP;
                 if (a < r && c < ncol) p.X[(long long)(c0 + c) * r + a] = Xn[c * LDN + a];
             }
-            for (int k = tid; k < RP * kUpdCols; k += kUpdThreads) {
-                int a = k / kUpdCols, c = k % kUpdCols;
-                if (a < r && c < ncol) p.Xb[(long long)a * p.ldb + c0 + c] = __float2bfloat16_rn(Xn[c * LDN + a]);
-            }
+            if (p.Xb)
+                for (int k = tid; k < RP * kUpdCols; k += kUpdThreads) {
+                    int a = k / kUpdCols, c = k % kUpdCols;
+                    if (a < r && c < ncol) p.Xb[(long long)a * p.ldb + c0 + c] = __float2bfloat16_rn(Xn[c * LDN + a]);
+                }
         }
+        if (p.Xs)
+            for (int k = tid; k < RP * kUpdCols; k += kUpdThreads) {
+                const int c = k / RP, a = k % RP;
+                if (c < ncol) store_cut(p.Xs + (long long)(c0 + c) * RP + a, p.part, Xn[c * LDN + a]);
+            }
     }
     // partial Gram of the new tile: rows ga*TA.., columns gb*TA.. (columns outside ncol are zero)
     {
@@ -2370,7 +2416,8 @@ struct KlUpdParams {
     int r, cols, npad;
     float eps;
     int update;
-    int additive;        // 1: X = max(0, X + (X / max(sum, eps)) (num - sum))
+    int additive;        // 1: X = max(0, X + (X / max(sum, eps)) (num - sum)); 2: num has the - sum already
+    long long part;      // FP32 products (Xb null): Xr holds the three parts of X, this far apart
 };
 
 // COLS columns of H (rows of W) per CTA: 8 for the H-step (its m is the smaller side: more CTAs),
@@ -2463,7 +2510,7 @@ __global__ void __launch_bounds__(kUpdThreads) tc_kl_update_kernel(KlUpdParams p
             if (a < r && c < ncol) {
                 float x = Xs[a * LDX + c];
                 if (p.additive) {
-                    x = x + (x / sumS[a]) * (acc[j] - sumR[a]);
+                    x = x + (x / sumS[a]) * (p.additive == 1 ? acc[j] - sumR[a] : acc[j]);
                     x = x < 0.f ? 0.f : x;
                 } else {
                     x *= (acc[j] / sumS[a]);
@@ -2483,13 +2530,17 @@ __global__ void __launch_bounds__(kUpdThreads) tc_kl_update_kernel(KlUpdParams p
                 if (a < r && c < ncol) p.X[(long long)(c0 + c) * r + a] = Xs[a * LDX + c];
             }
         }
-        for (int k = tid; k < RP * COLS; k += kUpdThreads) {  // Xb: c fastest
-            const int a = k / COLS, c = k % COLS;
-            if (a < r && c < ncol) p.Xb[(long long)a * p.ldb + c0 + c] = __float2bfloat16_rn(Xs[a * LDX + c]);
-        }
+        if (p.Xb)
+            for (int k = tid; k < RP * COLS; k += kUpdThreads) {  // Xb: c fastest
+                const int a = k / COLS, c = k % COLS;
+                if (a < r && c < ncol) p.Xb[(long long)a * p.ldb + c0 + c] = __float2bfloat16_rn(Xs[a * LDX + c]);
+            }
         for (int k = tid; k < RP * COLS; k += kUpdThreads) {  // Xr: a fastest
             const int c = k / RP, a = k % RP;
-            if (c < ncol) p.Xr[(long long)(c0 + c) * p.ldr + a] = __float2bfloat16_rn(a < r ? Xs[a * LDX + c] : 0.f);
+            const float x = a < r ? Xs[a * LDX + c] : 0.f;
+            if (c >= ncol) continue;
+            if (p.Xb) p.Xr[(long long)(c0 + c) * p.ldr + a] = __float2bfloat16_rn(x);
+            else store_cut(p.Xr + (long long)(c0 + c) * p.ldr + a, p.part, x);
         }
     }
     if (tid < RP) {
@@ -3162,6 +3213,8 @@ static KlUpdParams kl_params_w(gpunmf_job *j, int update) {
     return u;
 }
 
+#include "split_f32.cuh"
+
 static gpunmf_status setup_quality(gpunmf_job *j);
 
 static gpunmf_status tc_create_kl(gpunmf_job *j) {
@@ -3585,12 +3638,14 @@ gpunmf_status tc_iterate(gpunmf_job *j, bool updateW) {
 }
 
 gpunmf_status tc_check(gpunmf_job *j) {
-    if (!j->tc || !j->tc->err) return GPUNMF_OK;
-    int e = 0;  // read in the job's stream order (its memory may be stream-ordered)
-    GPUNMF_CUDA_TRY(cudaMemcpyAsync(&e, j->tc->err, sizeof(int), cudaMemcpyDeviceToHost, j->stream));
+    const int *words[2] = {j->tc ? j->tc->err : nullptr, j->sp ? j->sp->err : nullptr};
+    int e[2] = {0, 0};  // read in the job's stream order (its memory may be stream-ordered)
+    if (!words[0] && !words[1]) return GPUNMF_OK;
+    for (int k = 0; k < 2; k++)
+        if (words[k]) GPUNMF_CUDA_TRY(cudaMemcpyAsync(&e[k], words[k], sizeof(int), cudaMemcpyDeviceToHost, j->stream));
     GPUNMF_CUDA_TRY(cudaStreamSynchronize(j->stream));
-    if (e != 0) {
-        set_error("tensor-core kernel gave up waiting (error bits 0x%x)", e);
+    if (e[0] | e[1]) {
+        set_error("tensor-core kernel gave up waiting (error bits 0x%x)", e[0] | e[1]);
         return GPUNMF_ERR_TIMEOUT;
     }
     return GPUNMF_OK;
