@@ -768,8 +768,8 @@ static void sp_layout(SpState *t, SpArena &a, int rule, int n, int m, int npad, 
     } else {
         a.get(&t->G_w, np * np);
         a.get(&t->G_h, np * np);
-        a.get(&t->GP_w, np * np * ceil_div(n, kUpdCols));
-        a.get(&t->GP_h, np * np * ceil_div(m, kUpdCols));
+        a.get(&t->GP_w, np * np * ceil_div(n, upd_rows(n, npad)));
+        a.get(&t->GP_h, np * np * ceil_div(m, upd_rows(m, npad)));
     }
     a.get(&t->P_h, (size_t)th->ctas * th->max_seg * kTileM * np);
     a.get(&t->P_w, (size_t)tw->ctas * tw->max_seg * kTileM * np);
@@ -972,8 +972,8 @@ gpunmf_status sp_create(gpunmf_job *j, bool residual_only) {
         t->gh.p.sum_partials = t->SP_w; t->gh.p.sum_out = t->S_w; t->gh.p.sum_count = ceil_div(n, kKlUpdColsW);
         t->gw.p.sum_partials = t->SP_h; t->gw.p.sum_out = t->S_h; t->gw.p.sum_count = ceil_div(m, kKlUpdColsH);
     } else {
-        t->gh.p.gram_partials = t->GP_w; t->gh.p.gram_out = t->G_w; t->gh.p.gram_count = ceil_div(n, kUpdCols);
-        t->gw.p.gram_partials = t->GP_h; t->gw.p.gram_out = t->G_h; t->gw.p.gram_count = ceil_div(m, kUpdCols);
+        t->gh.p.gram_partials = t->GP_w; t->gh.p.gram_out = t->G_w; t->gh.p.gram_count = ceil_div(n, upd_rows(n, t->npad));
+        t->gw.p.gram_partials = t->GP_h; t->gw.p.gram_out = t->G_h; t->gw.p.gram_count = ceil_div(m, upd_rows(m, t->npad));
         t->gh.p.gram_entries = t->gw.p.gram_entries = (int)(np * np);
     }
     return st;
@@ -996,12 +996,12 @@ static cudaError_t sp_update(gpunmf_job *j, bool is_w, int update) {
     UpdParams u{};
     u.X = is_w ? j->W : j->H; u.Xs = is_w ? t->Ws : t->Hs; u.part = (long long)rows * t->npad;
     u.ldx = j->n; u.G = is_w ? t->G_h : t->G_w; u.P = is_w ? t->P_w : t->P_h;
-    u.slot_ptr = g.slot_ptr; u.slot_list = g.slot_list; u.tile_slots = g.tile_slots;
+    u.slot_ptr = g.slot_ptr; u.slot_list = g.slot_list; u.is_w = is_w;
     u.gram_partials = is_w ? t->GP_w : t->GP_h;
     u.r = j->r; u.cols = rows; u.npad = t->npad; u.eps = j->eps; u.update = update;
     u.additive = rule_is_additive(j->rule);
     u.V = j->V; u.F = is_w ? j->H : j->W; u.K = is_w ? j->m : j->n;
-    return launch_update(u, t->npad, is_w, j->stream);
+    return launch_update(u, t->npad, j->stream);
 }
 
 static cudaError_t sp_cut_factors(gpunmf_job *j) {

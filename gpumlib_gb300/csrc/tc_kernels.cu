@@ -71,6 +71,7 @@ struct SkParams {
     float *gram_out;
     int gram_count;
     int gram_entries;
+    int ctas;  // without a fused update: CTAs that share the product; any more of the grid finish the Gram
     // fused update (kernel template FNP > 0).  Every CTA owns a contiguous slice of the rows of the
     // factor X it updates.  While its tensor pipe streams V, two worker warps assemble the Gram of
     // the other factor from that factor's per-CTA partials (each CTA sums a slice, then all copy
@@ -719,6 +720,31 @@ __device__ __forceinline__ float lg2_approx(float x) {
     return y;
 }
 
+// This CTA's entries [c*E/G, (c+1)*E/G) of the Gram matrix, by nt threads: four lanes share an entry and
+// sum the partials in a fixed order, whatever nt and G are.
+__device__ __forceinline__ void finish_gram(const SkParams &p, int et, int nt) {
+    const long long E = p.gram_entries;
+    const long long e0 = (long long)blockIdx.x * E / gridDim.x, e1 = (long long)(blockIdx.x + 1) * E / gridDim.x;
+    for (long long eb = e0; eb < e1; eb += nt / 4) {
+        const long long e = eb + (et >> 2);
+        float s = 0.f;
+        if (e < e1) {
+            int z = et & 3;
+            for (; z + 28 < p.gram_count; z += 32) {
+                float v[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[q] = p.gram_partials[(size_t)(z + 4 * q) * E + e];
+#pragma unroll
+                for (int q = 0; q < 8; q++) s += v[q];
+            }
+            for (; z < p.gram_count; z += 4) s += p.gram_partials[(size_t)z * E + e];
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        if (e < e1 && (et & 3) == 0) p.gram_out[e] = s;
+    }
+}
+
 // QF: the H-step also samples the quality of the factors it starts from (the value
 // NMF::DetermineQualityImprovement reads, nmf_base.h:70-89), on the V tiles it streams anyway:
 // per block (128 columns u of V x 128 rows i) one more MMA forms S = H' W over the block
@@ -757,9 +783,16 @@ __global__ void __launch_bounds__(gemm_threads(FNP, QF), 1)
     const uint32_t tcols = QF ? 512u : p.tmem_cols;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ctas = FNP ? (int)gridDim.x : p.ctas;
+    if (FNP == 0 && (int)blockIdx.x >= ctas) {  // no blocks of the product: a share of the Gram only
+        griddep_wait();
+        griddep_launch_dependents();
+        if (p.gram_out) finish_gram(p, threadIdx.x, kGemmThreads);
+        return;
+    }
     const long long T = (long long)p.tiles * p.kblocks;
-    const long long lo = (long long)blockIdx.x * T / gridDim.x;
-    const long long hi = (long long)(blockIdx.x + 1) * T / gridDim.x;
+    const long long lo = (long long)blockIdx.x * T / ctas;
+    const long long hi = (long long)(blockIdx.x + 1) * T / ctas;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; s++) {
@@ -958,32 +991,9 @@ __global__ void __launch_bounds__(gemm_threads(FNP, QF), 1)
     } else if (warp < 6) {
         griddep_wait();
         griddep_launch_dependents();
-        // While the first accumulator fills, finish the Gram matrix the update kernel of the
-        // previous half-step left as per-CTA partials: this CTA owns entries
-        // [c*E/G, (c+1)*E/G); four lanes share an entry and sum the partials in a fixed order.
-        if (FNP == 0 && p.gram_out) {
-            const int et = threadIdx.x - 64;  // 0..127
-            const long long E = p.gram_entries;
-            const long long e0 = (long long)blockIdx.x * E / gridDim.x, e1 = (long long)(blockIdx.x + 1) * E / gridDim.x;
-            for (long long eb = e0; eb < e1; eb += 32) {
-                const long long e = eb + (et >> 2);
-                float s = 0.f;
-                if (e < e1) {
-                    int z = et & 3;
-                    for (; z + 28 < p.gram_count; z += 32) {
-                        float v[8];
-#pragma unroll
-                        for (int q = 0; q < 8; q++) v[q] = p.gram_partials[(size_t)(z + 4 * q) * E + e];
-#pragma unroll
-                        for (int q = 0; q < 8; q++) s += v[q];
-                    }
-                    for (; z < p.gram_count; z += 4) s += p.gram_partials[(size_t)z * E + e];
-                }
-                s += __shfl_xor_sync(0xffffffffu, s, 1);
-                s += __shfl_xor_sync(0xffffffffu, s, 2);
-                if (e < e1 && (et & 3) == 0) p.gram_out[e] = s;
-            }
-        }
+        // while the first accumulator fills, finish this CTA's share of the Gram matrix that the update
+        // kernel of the previous half-step left as partials
+        if (FNP == 0 && p.gram_out) finish_gram(p, threadIdx.x - 64, 128);
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         int acc = 0, seg = 0;
@@ -1505,6 +1515,14 @@ __device__ __forceinline__ void cut3(float x, uint32_t &p0, uint32_t &p1, uint32
 }
 // the top halves of two words, the first one's in the low half
 __device__ __forceinline__ uint32_t pack_top(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x7632); }
+// the parts of two neighbours
+__device__ __forceinline__ void store_cut2(__nv_bfloat16 *dst, long long part, float x, float y) {
+    uint32_t a[3], b[3];
+    cut3(x, a[0], a[1], a[2]);
+    cut3(y, b[0], b[1], b[2]);
+#pragma unroll
+    for (int q = 0; q < 3; q++) *reinterpret_cast<uint32_t *>(dst + q * part) = pack_top(a[q], b[q]);
+}
 __device__ __forceinline__ void store_cut(__nv_bfloat16 *dst, long long part, float x) {
     uint32_t p0, p1, p2;
     cut3(x, p0, p1, p2);
@@ -1516,19 +1534,21 @@ __device__ __forceinline__ void store_cut(__nv_bfloat16 *dst, long long part, fl
 
 // ------------------------------------------------------------------------
 // update kernel (FP32): the multiplicative rule of nmf_kernels.cu:43-47 (or the
-// additive rule of nmf_kernels.cu:31-38) on an
-// r x 32 tile X of the factor being updated, with
-//   H-step: X = H(:, u0:u0+32),   den = G_W X          (G_W = W'W)
-//   W-step: X = W(i0:i0+32, :)',  den = G_H X = (X' G_H)'  (G_H = H H', symmetric)
-// The numerator is the sum of the GEMM's partial slots for the tile (fixed
-// order).  The kernel writes X (FP32), its BF16 copy for the next GEMM, and
-// this CTA's partial Gram X X' (r x r) that the next GEMM's epilogue warps
-// reduce.  256 threads as a 16 x 16 grid; RP = r rounded up to 16, so each
-// thread owns RP/16 rows of the tile.
+// additive rule of nmf_kernels.cu:31-38) on ROWS rows X of the factor being updated (columns u of H
+// or rows i of W), with den = X G, G the other factor's r x r Gram (symmetric).
+// The numerator is the sum of the GEMM's partial slots for the tile, in their order.  The kernel
+// writes X (FP32), its BF16 copy (or, for the FP32 products, its three parts) for the next GEMM, and
+// this CTA's partial Gram X'X (r x r) that the next GEMM reduces.  256 threads as a 16 x 16 grid;
+// RP = r rounded up to 16, so a thread owns RP / 16 columns of ROWS / 16 rows.
+//
+// Bound: latency for few rows; else the r x r matrices that every CTA reads (G) and writes (its
+// partial, which the GEMM reads again), so the more rows a CTA the better while the SMs stay
+// occupied: upd_rows.  8192 x 8192, r = 128: 76 us a launch with 16 rows, about 20 with 64 (33 and 8 MB each
+// of G read and of partials written).
 // ------------------------------------------------------------------------
-constexpr int kUpdCols = 16;  // columns (H-step) or rows (W-step) per CTA; 16 x 16 threads
 constexpr int kUpdThreads = 256;
-constexpr int kSlotW = 8;  // width of the per-tile slot table (tiles with more slots use the CSR lists)
+constexpr int kUpdGramRows = 16;  // rows of a Gram partial of a BF16 job
+constexpr int kSlotW = 8;  // width of the KL update's per-tile slot table (tiles with more slots use the CSR lists)
 
 struct UpdParams {
     float *X;                 // FP32 factor (H column-major r x m, or W column-major n x r)
@@ -1538,10 +1558,10 @@ struct UpdParams {
     const float *G;           // r x r Gram for the denominator
     const float *P;           // GEMM partial slots [slot][128][npad]
     const int *slot_ptr, *slot_list;
-    const int *tile_slots;    // [tiles][kSlotW] slot ids, -1 padded; null when a tile has more slots
-    float *gram_partials;     // [cta][RP*RP]
+    float *gram_partials;     // [partial][RP*RP]
     int r, cols, npad;
     float eps;
+    int is_w;
     int update;               // 0: only write the Gram partials of X (initialisation)
     int additive;             // 1: X = max(0, X + (X / den) (num - den)) (nmf_kernels.cu:31-38)
     __nv_bfloat16 *Xs;        // FP32 products: the three parts of X instead of Xb, at part * q + c * RP + a
@@ -1552,228 +1572,257 @@ struct UpdParams {
 
 // A numerator of the FP32 products by plain FP32 fused multiply-adds, where the sum of the parts'
 // products is not finite: a part of an infinity or NaN has lost which of the two it was.
-template <bool IS_W>
 __device__ __noinline__ float plain_sum(const UpdParams &p, int row, int a) {
     float s = 0.f;
     for (int k = 0; k < p.K; k++)
-        s = IS_W ? fmaf(p.V[(long long)k * p.cols + row], p.F[(long long)k * p.r + a], s)
+        s = p.is_w ? fmaf(p.V[(long long)k * p.cols + row], p.F[(long long)k * p.r + a], s)
                  : fmaf(p.V[(long long)row * p.K + k], p.F[(long long)a * p.K + k], s);
     return s;
 }
 
-template <int RP, bool IS_W>
-__global__ void __launch_bounds__(kUpdThreads) tc_update_kernel(UpdParams p) {
-    constexpr int TA = RP / 16;
-    constexpr int LDX = kUpdCols + 1;
-    extern __shared__ float sm[];
-    float *Gs = sm;                  // [RP][RP], zero outside r
-    float *Xs = Gs + RP * RP;        // [RP][LDX]  X(a, c)
-    float *Ns = Xs + RP * LDX;       // [RP][LDX]  numerators, later the new X as [c][RP + 4]
+// Rows per CTA and its threads.  Up to rank 64: 16 rows, 256 threads; several CTAs of an SM overlap their
+// latencies (8192 x 8192, r = 64, an iteration: 16 rows 131 us, 32 132, 64 152).  Above, every CTA's
+// r x r matrices weigh more: 64 rows and 512 threads where that still makes about one CTA for every
+// other SM (r = 128, an iteration: 8192 rows 64 / 32 / 16 193 / 224 / 307 us, 4000 rows 108 / 100; the
+// factors' odd multiples of 16, read one value at a time: 3000 rows of r = 80 62 / 65), else 32 rows
+// with 512 threads, or 256 for the odd multiples (500 rows, r = 100: 55 us against 74).  Above rank
+// 128 G leaves room for 32 rows only.
+__host__ __device__ constexpr bool upd_odd(int rp) { return rp / 16 % 2 != 0; }
+__host__ __device__ constexpr int upd_rows(int rows, int rp) {
+    return rp <= 64 ? 16 : rp <= 128 && rows > (upd_odd(rp) ? 2048 : 32 * kNumSMsGB300) ? 64 : 32;
+}
+__host__ __device__ constexpr int upd_threads(int rp, int cta_rows) {
+    return rp > 64 && rp <= 128 && (cta_rows == 64 || !upd_odd(rp)) ? 512 : 256;
+}
+
+// A thread's columns of the rank: vectors of four (or two) 16 vectors apart, so that the 16 threads of a
+// row read neighbouring vectors
+__host__ __device__ constexpr int upd_vec(int ta) { return ta % 4 == 0 ? 4 : ta % 2 == 0 ? 2 : 1; }
+template <int TA>
+__device__ __forceinline__ int upd_col(int g, int i) {
+    constexpr int V = upd_vec(TA);
+    return (g + 16 * (i / V)) * V + i % V;
+}
+template <int TA>
+__device__ __forceinline__ void upd_lds(const float *row, int g, float (&v)[TA]) {
+    constexpr int V = upd_vec(TA);
+#pragma unroll
+    for (int i = 0; i < TA; i += V) lds_vec<V>(row + upd_col<TA>(g, i), *reinterpret_cast<float (*)[V]>(&v[i]));
+}
+
+template <int RP, int ROWS>
+__global__ void __launch_bounds__(upd_threads(RP, ROWS)) tc_update_kernel(UpdParams p) {
+    constexpr int NT = upd_threads(RP, ROWS);
+    constexpr int TA = RP / 16, RT = ROWS * 16 / NT;
+    constexpr int LDX = ROWS + 4, LDN = RP + 4;
+    extern __shared__ __align__(16) float sm[];
+    float *Gs = sm;               // [RP][RP], zero outside r
+    float *Xs = Gs + RP * RP;     // [RP][LDX]  the old X(a, row)
+    float *Ns = Xs + RP * LDX;    // [ROWS][LDN]  numerators, then the new X
     const int tid = threadIdx.x;
-    const int c0 = blockIdx.x * kUpdCols;
-    const int ncol = min(kUpdCols, p.cols - c0);
+    const int c0 = blockIdx.x * ROWS;
+    const int ncol = min(ROWS, p.cols - c0);
     const int r = p.r;
     griddep_wait();  // the GEMM's partial slots and Gram are complete
     griddep_launch_dependents();
-    // Shared-memory fills: every thread first issues all of its loads (compile-time trip counts,
-    // fully unrolled), then stores, so the loads of a thread are in flight together.
-    // X tile (zero outside r rows / ncol columns)
-    constexpr int XL = RP * kUpdCols / kUpdThreads;
-    {
-        float xv[XL];
+    // the old rows, zero outside r and ncol; a thread issues up to sixteen loads before it stores
+    constexpr int XL = RP * ROWS / NT, XB = XL < 16 ? XL : 16;
+#pragma unroll 1
+    for (int j0 = 0; j0 < XL; j0 += XB) {
+        float xv[XB];
+        int at[XB];
 #pragma unroll
-        for (int j = 0; j < XL; j++) {
-            const int k = tid + j * kUpdThreads;
-            if (IS_W) {
-                const int a = k / kUpdCols, c = k % kUpdCols;
-                xv[j] = (a < r && c < ncol) ? p.X[(long long)a * p.ldx + c0 + c] : 0.f;
-            } else {
-                const int c = k / RP, a = k % RP;
-                xv[j] = (a < r && c < ncol) ? p.X[(long long)(c0 + c) * r + a] : 0.f;
+        for (int j = 0; j < XB; j++) {
+            const int k = tid + (j0 + j) * NT;
+            xv[j] = 0.f;
+            at[j] = -1;
+            if (j0 + j < XL) {
+                if (p.is_w) {  // along W's columns
+                    const int a = k / ROWS, c = k % ROWS;
+                    if (a < r && c < ncol) xv[j] = p.X[(long long)a * p.ldx + c0 + c];
+                    at[j] = a * LDX + c;
+                } else {       // 8 of H's rank by 4 columns a warp step: whole sectors, distinct banks
+                    const int w = k >> 5, a = (w % (RP / 8)) * 8 + (k & 7), c = (w / (RP / 8)) * 4 + ((k >> 3) & 3);
+                    if (a < r && c < ncol) xv[j] = p.X[(long long)(c0 + c) * r + a];
+                    at[j] = a * LDX + c;
+                }
             }
         }
 #pragma unroll
-        for (int j = 0; j < XL; j++) {
-            const int k = tid + j * kUpdThreads;
-            if (IS_W) Xs[(k / kUpdCols) * LDX + k % kUpdCols] = xv[j];
-            else Xs[(k % RP) * LDX + k / RP] = xv[j];
-        }
-    }
-    if (p.update) {  // G is RP x RP (zero outside r x r: the rows of X beyond r are zero)
-        constexpr int GL = RP * RP / kUpdThreads;
-        constexpr int GC = GL < 16 ? GL : 16;
-#pragma unroll 1
-        for (int j0 = 0; j0 < GL; j0 += GC) {
-            float gv[GC];
-#pragma unroll
-            for (int j = 0; j < GC; j++) gv[j] = (j0 + j < GL) ? p.G[tid + (j0 + j) * kUpdThreads] : 0.f;
-#pragma unroll
-            for (int j = 0; j < GC; j++)
-                if (j0 + j < GL) Gs[tid + (j0 + j) * kUpdThreads] = gv[j];
-        }
+        for (int j = 0; j < XB; j++)
+            if (at[j] >= 0) Xs[at[j]] = xv[j];
     }
     if (p.update) {
-        // numerators: the tile's partial slots summed in slot order.  Rows lrow0 + c < 128 of a slot
-        // (RP == npad) are in bounds for every c < kUpdCols, so the loads need no column guard (the
-        // sums over the tile's padding rows are never stored).  The table lists a tile's slots
-        // first, then -1: four slots' loads are issued together (an absent slot reads the first one
-        // again and is not added); a branch around each slot's loads would serialise them.
+        // G (RP x RP; the rows of X beyond r are zero)
+        constexpr int G4 = RP * RP / 4;
+#pragma unroll 4
+        for (int k = tid; k < G4; k += NT)
+            reinterpret_cast<float4 *>(Gs)[k] = __ldcg(reinterpret_cast<const float4 *>(p.G) + k);
+        // numerators: the tile's slots summed in their order, four slots' loads of a thread together.
+        // (Rows of a slot beyond the last are in bounds, the tile has 128; they are never stored.)
         const int tile = c0 / 128, lrow0 = c0 % 128;
-        constexpr int PER = kUpdCols * RP / kUpdThreads;
-        float acc[PER];
-#pragma unroll
-        for (int j = 0; j < PER; j++) acc[j] = 0.f;
-        if (p.tile_slots) {
-            const int4 *ts = reinterpret_cast<const int4 *>(p.tile_slots + (size_t)tile * kSlotW);
-            const int4 sa = ts[0], sb = ts[1];
-            const int sl[kSlotW] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
-#pragma unroll
-            for (int q0 = 0; q0 < kSlotW; q0 += 4) {
-                if (q0 > 0 && sl[q0] < 0) continue;
-                float v[4][PER];
+        const int s0 = p.slot_ptr[tile], s1 = p.slot_ptr[tile + 1];
+        constexpr int N4 = ROWS * RP / 4;
+#pragma unroll 1
+        for (int k0 = 0; k0 < N4; k0 += 2 * NT) {
+            const int ka = k0 + tid, kb = ka + NT;
+            const bool oa = ka < N4, ob = kb < N4;
+            float4 sa = make_float4(0.f, 0.f, 0.f, 0.f), sb = sa;
+            auto add = [](float4 &s, const float4 &v) { s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; };
+#pragma unroll 1
+            for (int q0 = s0; q0 < s1; q0 += 4) {
+                float4 va[4], vb[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const int sq = sl[q0 + q] >= 0 ? sl[q0 + q] : sl[0];
-                    const float *base = p.P + ((size_t)sq * 128 + lrow0) * p.npad;
-#pragma unroll
-                    for (int j = 0; j < PER; j++) {
-                        const int k = tid + j * kUpdThreads, c = k / RP, a = k % RP;
-                        v[q][j] = base[c * p.npad + a];
-                    }
+                    const int slot = p.slot_list[min(q0 + q, s1 - 1)];
+                    const float4 *src = reinterpret_cast<const float4 *>(p.P + ((size_t)slot * 128 + lrow0) * RP);
+                    if (oa) va[q] = __ldcg(src + ka);
+                    if (ob) vb[q] = __ldcg(src + kb);
                 }
 #pragma unroll
                 for (int q = 0; q < 4; q++)
-                    if (sl[q0 + q] >= 0) {
-#pragma unroll
-                        for (int j = 0; j < PER; j++) acc[j] += v[q][j];
+                    if (q0 + q < s1) {
+                        if (oa) add(sa, va[q]);
+                        if (ob) add(sb, vb[q]);
                     }
             }
-        } else {
-            const int s0 = p.slot_ptr[tile], s1 = p.slot_ptr[tile + 1];
-            for (int q = s0; q < s1; q++) {
-                const float *base = p.P + ((size_t)p.slot_list[q] * 128 + lrow0) * p.npad;
-#pragma unroll
-                for (int j = 0; j < PER; j++) {
-                    const int k = tid + j * kUpdThreads, c = k / RP, a = k % RP;
-                    if (c < ncol) acc[j] += base[c * p.npad + a];
+            auto put = [&](int k, float4 v) {
+                const int c = k / (RP / 4), a = (k % (RP / 4)) * 4;
+                const float inf = __int_as_float(0x7F800000);
+                if (p.Xs && c < ncol && !(fabsf(v.x) < inf && fabsf(v.y) < inf && fabsf(v.z) < inf && fabsf(v.w) < inf)) {
+                    if (!(fabsf(v.x) < inf) && a < r) v.x = plain_sum(p, c0 + c, a);
+                    if (!(fabsf(v.y) < inf) && a + 1 < r) v.y = plain_sum(p, c0 + c, a + 1);
+                    if (!(fabsf(v.z) < inf) && a + 2 < r) v.z = plain_sum(p, c0 + c, a + 2);
+                    if (!(fabsf(v.w) < inf) && a + 3 < r) v.w = plain_sum(p, c0 + c, a + 3);
                 }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < PER; j++) {
-            const int k = tid + j * kUpdThreads, c = k / RP, a = k % RP;
-            if (p.Xs && !(fabsf(acc[j]) < __int_as_float(0x7F800000)) && a < r && c < ncol)
-                acc[j] = plain_sum<IS_W>(p, c0 + c, a);
-            Ns[a * LDX + c] = acc[j];
+                *reinterpret_cast<float4 *>(Ns + c * LDN + a) = v;
+            };
+            if (oa) put(ka, sa);
+            if (ob) put(kb, sb);
         }
     }
     __syncthreads();
     const int ga = tid & 15, gc = tid >> 4;
-    constexpr int CPT = kUpdCols / 16;  // columns per thread
-    float *Xn = Ns;  // reused as [c][RP + 4] once the numerators are in registers
-    constexpr int LDN = RP + 4;
     if (p.update) {
-        // den(a, c) for a in ga*TA.., c in gc*CPT..
-        float den[TA][CPT];
+        float den[TA][RT];
 #pragma unroll
         for (int i = 0; i < TA; i++)
 #pragma unroll
-            for (int j = 0; j < CPT; j++) den[i][j] = 0.f;
+            for (int j = 0; j < RT; j++) den[i][j] = 0.f;
+#pragma unroll 4
         for (int b = 0; b < RP; b++) {
-            float xb[CPT];
-#pragma unroll
-            for (int j = 0; j < CPT; j++) xb[j] = Xs[b * LDX + gc * CPT + j];
-#pragma unroll
-            for (int i = 0; i < TA; i++) {
-                float g = Gs[b * RP + ga * TA + i];
-#pragma unroll
-                for (int j = 0; j < CPT; j++) den[i][j] = fmaf(g, xb[j], den[i][j]);
-            }
-        }
-        float nv[TA][CPT], xv[TA][CPT];
-#pragma unroll
-        for (int i = 0; i < TA; i++)
-#pragma unroll
-            for (int j = 0; j < CPT; j++) {
-                nv[i][j] = Ns[(ga * TA + i) * LDX + gc * CPT + j];
-                xv[i][j] = Xs[(ga * TA + i) * LDX + gc * CPT + j];
-            }
-        __syncthreads();  // everyone has read Ns and Xs
-#pragma unroll
-        for (int i = 0; i < TA; i++)
-#pragma unroll
-            for (int j = 0; j < CPT; j++) {
-                int a = ga * TA + i;
-                float x = xv[i][j];
-                if (a < r && gc * CPT + j < ncol) {  // outside stays 0 (the additive step has no eps)
-                    if (p.additive) {
-                        x = x + (x / den[i][j]) * (nv[i][j] - den[i][j]);
-                        x = x < 0.f ? 0.f : x;
-                    } else {
-                        x *= nv[i][j] / (den[i][j] + p.eps);
-                    }
-                }
-                Xn[(gc * CPT + j) * LDN + a] = x;
-            }
-    } else {
-        for (int k = tid; k < RP * kUpdCols; k += kUpdThreads) {
-            int c = k / RP, a = k % RP;
-            Xn[c * LDN + a] = Xs[a * LDX + c];
-        }
-    }
-    __syncthreads();
-    if (p.update) {
-        if (IS_W) {
-            for (int k = tid; k < RP * kUpdCols; k += kUpdThreads) {
-                int a = k / kUpdCols, c = k % kUpdCols;
-                if (a < r && c < ncol) {
-                    float x = Xn[c * LDN + a];
-                    p.X[(long long)a * p.ldx + c0 + c] = x;
-                    if (p.Xb) p.Xb[(long long)a * p.ldb + c0 + c] = __float2bfloat16_rn(x);
-                }
-            }
-        } else {
-            for (int k = tid; k < RP * kUpdCols; k += kUpdThreads) {
-                int c = k / RP, a = k % RP;
-                if (a < r && c < ncol) p.X[(long long)(c0 + c) * r + a] = Xn[c * LDN + a];
-            }
-            if (p.Xb)
-                for (int k = tid; k < RP * kUpdCols; k += kUpdThreads) {
-                    int a = k / kUpdCols, c = k % kUpdCols;
-                    if (a < r && c < ncol) p.Xb[(long long)a * p.ldb + c0 + c] = __float2bfloat16_rn(Xn[c * LDN + a]);
-                }
-        }
-        if (p.Xs)
-            for (int k = tid; k < RP * kUpdCols; k += kUpdThreads) {
-                const int c = k / RP, a = k % RP;
-                if (c < ncol) store_cut(p.Xs + (long long)(c0 + c) * RP + a, p.part, Xn[c * LDN + a]);
-            }
-    }
-    // partial Gram of the new tile: rows ga*TA.., columns gb*TA.. (columns outside ncol are zero)
-    {
-        const int gb = tid >> 4;
-        float acc[TA][TA];
-#pragma unroll
-        for (int i = 0; i < TA; i++)
-#pragma unroll
-            for (int k = 0; k < TA; k++) acc[i][k] = 0.f;
-        for (int c = 0; c < kUpdCols; c++) {
-            float xa[TA], xb[TA];
-#pragma unroll
-            for (int i = 0; i < TA; i++) {
-                xa[i] = Xn[c * LDN + ga * TA + i];
-                xb[i] = Xn[c * LDN + gb * TA + i];
-            }
+            float xb[RT], g[TA];
+            lds_vec<RT>(Xs + b * LDX + gc * RT, xb);
+            upd_lds<TA>(Gs + b * RP, ga, g);
 #pragma unroll
             for (int i = 0; i < TA; i++)
 #pragma unroll
-                for (int k = 0; k < TA; k++) acc[i][k] = fmaf(xa[i], xb[k], acc[i][k]);
+                for (int j = 0; j < RT; j++) den[i][j] = fmaf(g[i], xb[j], den[i][j]);
         }
-        float *out = p.gram_partials + (size_t)blockIdx.x * RP * RP;
 #pragma unroll
-        for (int i = 0; i < TA; i++)
+        for (int i = 0; i < TA; i++) {
+            const int a = upd_col<TA>(ga, i);
 #pragma unroll
-            for (int k = 0; k < TA; k++) out[(ga * TA + i) * RP + gb * TA + k] = acc[i][k];
+            for (int j = 0; j < RT; j++) {
+                const int c = gc * RT + j;
+                float *at = Ns + c * LDN + a;  // this thread's alone
+                const float nv = *at;
+                float x = Xs[a * LDX + c];
+                if (a < r && c < ncol) {  // outside stays 0 (the additive step has no eps)
+                    if (p.additive) {
+                        x = x + (x / den[i][j]) * (nv - den[i][j]);
+                        x = x < 0.f ? 0.f : x;
+                    } else {
+                        x *= nv / (den[i][j] + p.eps);
+                    }
+                } else {
+                    x = 0.f;
+                }
+                *at = x;
+            }
+        }
+        __syncthreads();
+        // X and the BF16 copy along their columns: a warp step covers 32 rows of four columns (16 of
+        // eight), lane l row l, the column rotating with l / 8 and the step (bank conflicts)
+        constexpr int RW = ROWS < 32 ? ROWS : 32, CW = 128 / RW;
+        if (p.is_w || p.Xb) {
+#pragma unroll 4
+            for (int k = tid; k < RP * ROWS; k += NT) {
+                const int lane = k & 31, st = (k >> 5) & 3, patch = k >> 7;
+                const int c = RW * (patch % (ROWS / RW)) + (lane & (RW - 1));
+                const int a = CW * (patch / (ROWS / RW)) + (CW == 4 ? ((lane >> 3) + st) & 3 : 2 * (((lane >> 2) + st) & 3) + (lane >> 4));
+                if (a < r && c < ncol) {
+                    const float x = Ns[c * LDN + a];
+                    if (p.is_w) p.X[(long long)a * p.ldx + c0 + c] = x;
+                    if (p.Xb) p.Xb[(long long)a * p.ldb + c0 + c] = __float2bfloat16_rn(x);
+                }
+            }
+        }
+        if (!p.is_w)
+            for (int k = tid; k < RP * ROWS; k += NT) {
+                const int c = k / RP, a = k % RP;
+                if (a < r && c < ncol) p.X[(long long)(c0 + c) * r + a] = Ns[c * LDN + a];
+            }
+        if (p.Xs)
+            for (int k = tid; k < RP * ROWS / 2; k += NT) {  // two values of a row
+                const int c = k / (RP / 2), a = k % (RP / 2) * 2;
+                if (c < ncol) store_cut2(p.Xs + (long long)(c0 + c) * RP + a, p.part, Ns[c * LDN + a], Ns[c * LDN + a + 1]);
+            }
+    } else {
+        for (int k = tid; k < RP * ROWS; k += NT) {
+            const int c = k / RP, a = k % RP;
+            Ns[c * LDN + a] = Xs[a * LDX + c];
+        }
+        __syncthreads();
+    }
+    // partial Gram of the new rows (those outside ncol are zero), 256 threads with a TA x TA block each.
+    // BF16 jobs: one for every 16 rows (a sum over more rows at once would round differently, and the
+    // BF16 copies carry the last bits on); a second half of the threads takes the second half of the
+    // groups.  FP32 products: one for all rows, the second half's sums added through G's place.
+    {
+        constexpr int H = NT / 256;
+        const int half = tid >> 8, gb = gc & 15;
+        const int step = p.Xs ? ROWS / H : 16;
+#pragma unroll 1
+        for (int c1 = half * (ROWS / H); c1 < (half + 1) * (ROWS / H); c1 += step) {
+            float acc[TA][TA];
+#pragma unroll
+            for (int i = 0; i < TA; i++)
+#pragma unroll
+                for (int k = 0; k < TA; k++) acc[i][k] = 0.f;
+#pragma unroll 2
+            for (int c = c1; c < c1 + step; c++) {
+                float xa[TA], xb[TA];
+                upd_lds<TA>(Ns + c * LDN, ga, xa);
+                upd_lds<TA>(Ns + c * LDN, gb, xb);
+#pragma unroll
+                for (int i = 0; i < TA; i++)
+#pragma unroll
+                    for (int k = 0; k < TA; k++) acc[i][k] = fmaf(xa[i], xb[k], acc[i][k]);
+            }
+            if (H == 2 && p.Xs) {  // (G is read by no one any more: a barrier lies behind the denominators)
+                if (half == 1) {
+#pragma unroll
+                    for (int i = 0; i < TA; i++)
+#pragma unroll
+                        for (int k = 0; k < TA; k++) Gs[(i * TA + k) * 256 + (tid & 255)] = acc[i][k];
+                }
+                __syncthreads();
+                if (half == 1) return;
+#pragma unroll
+                for (int i = 0; i < TA; i++)
+#pragma unroll
+                    for (int k = 0; k < TA; k++) acc[i][k] += Gs[(i * TA + k) * 256 + tid];
+            }
+            const int part = p.Xs ? blockIdx.x : blockIdx.x * (ROWS / 16) + c1 / 16;
+            if (p.Xs || c1 < ncol) {
+                float *out = p.gram_partials + (size_t)part * RP * RP;
+#pragma unroll
+                for (int i = 0; i < TA; i++)
+#pragma unroll
+                    for (int k = 0; k < TA; k++) out[upd_col<TA>(gb, k) * RP + upd_col<TA>(ga, i)] = acc[i][k];
+            }
+        }
     }
 }
 
@@ -2574,7 +2623,6 @@ struct TcGemm {
     int smem_qf = 0;  // shared memory of the variant with the quality warps
     int fnp = 0;  // fused update rank (kernel template argument), 0 = separate update kernel
     int *slot_ptr = nullptr, *slot_list = nullptr;
-    int *tile_slots = nullptr;
     int *counters = nullptr;  // [tiles] arrivals, [tiles] readers done, [tiles] readers, [2] Gram assembly
     float *grams = nullptr;   // [grid][npad^2] per-CTA Gram partials of the factor this GEMM updates
 };
@@ -2744,15 +2792,6 @@ static gpunmf_status setup_gemm(gpunmf_job *j, TcGemm &g, int rows, int K, int n
     std::vector<int> ptr, list;
     int max_seg = 1;
     schedule(tiles, kblocks, g.grid, &max_seg, ptr, list);
-    bool table_ok = true;
-    for (int t = 0; t < tiles; t++)
-        if (ptr[t + 1] - ptr[t] > kSlotW) table_ok = false;
-    std::vector<int> table;
-    if (table_ok) {
-        table.assign((size_t)tiles * kSlotW, -1);
-        for (int t = 0; t < tiles; t++)
-            for (int q = ptr[t]; q < ptr[t + 1]; q++) table[(size_t)t * kSlotW + (q - ptr[t])] = list[q];
-    }
     const int stage_bytes = bps * (kStageABytes + boxB);
     int stages = std::min(kMaxStages, (budget - 1024 - 256) / stage_bytes);
     // the fused kernel: at most three stages (96 KB of V per SM in flight).  More than that does not
@@ -2771,20 +2810,20 @@ static gpunmf_status setup_gemm(gpunmf_job *j, TcGemm &g, int rows, int K, int n
     g.p.tmem_cols = cols;
     g.p.err = err;
     g.p.wait_limit = kWaitLimitCycles;
+    // Where the product makes few CTAs, more of them share the Gram's npad^2 entries: 500 x 500, r = 100,
+    // took 22.7 us a launch with the product's 16 CTAs alone (the Gram 15 of them).
+    g.p.ctas = g.grid;
+    if (!fnp) g.grid = std::max(g.grid, std::min(j->tc->max_ctas, npad * npad / (kGemmThreads / 4)));
     g.smem = 1024 + stages * stage_bytes + (2 * stages + 5) * 8 + 16 + (fnp ? 16 + fused_smem_bytes(fnp) : 0);
     // with the folded quality sample: two H-tile slots, eight more barriers, the warps' sums
     g.smem_qf = g.smem + 2 * 2 * npad * kBlockK * 2 + (4 + 2 * kQfSBufs) * 8 + 2 * kQfWarps * 8;
     g.fnp = fnp;
-    size_t slots = (size_t)g.grid * max_seg;
+    size_t slots = (size_t)g.p.ctas * max_seg;
     cudaError_t e = job_dev_alloc(j, (void **)partials, slots * kTileM * npad * sizeof(float));
     if (e == cudaSuccess) e = job_dev_alloc(j, (void **)&g.slot_ptr, ptr.size() * sizeof(int));
     if (e == cudaSuccess) e = job_dev_alloc(j, (void **)&g.slot_list, std::max<size_t>(1, list.size()) * sizeof(int));
     if (e == cudaSuccess) e = job_h2d(j, g.slot_ptr, ptr.data(), ptr.size() * sizeof(int));
     if (e == cudaSuccess && !list.empty()) e = job_h2d(j, g.slot_list, list.data(), list.size() * sizeof(int));
-    if (e == cudaSuccess && table_ok) {
-        e = job_dev_alloc(j, (void **)&g.tile_slots, table.size() * sizeof(int));
-        if (e == cudaSuccess) e = job_h2d(j, g.tile_slots, table.data(), table.size() * sizeof(int));
-    }
     if (e != cudaSuccess) {
         set_error("tensor-core workspace allocation failed: %s", cudaGetErrorString(e));
         cudaGetLastError();
@@ -2882,19 +2921,21 @@ static cudaError_t set_gemm_smem_once() {
     return result;
 }
 
-static int update_smem_bytes(int rp) {
-    int ns = std::max(rp * (kUpdCols + 1), kUpdCols * (rp + 4));
-    return (rp * rp + rp * (kUpdCols + 1) + ns) * (int)sizeof(float);
+static int update_smem_bytes(int rp, int rows) {
+    return (rp * rp + rp * (rows + 4) + rows * (rp + 4)) * (int)sizeof(float);
 }
 
 template <int RP>
 static cudaError_t set_update_smem_rp() {
-    cudaError_t e = cudaFuncSetAttribute(tc_update_kernel<RP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         update_smem_bytes(RP));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(tc_update_kernel<RP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 update_smem_bytes(RP));
-    return e;
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if constexpr (RP <= 64) {
+        return cudaFuncSetAttribute(tc_update_kernel<RP, 16>, attr, update_smem_bytes(RP, 16));
+    } else {
+        cudaError_t e = cudaFuncSetAttribute(tc_update_kernel<RP, 32>, attr, update_smem_bytes(RP, 32));
+        if constexpr (RP <= 128)
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(tc_update_kernel<RP, 64>, attr, update_smem_bytes(RP, 64));
+        return e;
+    }
 }
 
 static cudaError_t set_update_smem(int rp) {
@@ -2908,13 +2949,23 @@ static cudaError_t set_update_smem(int rp) {
     return cudaErrorInvalidValue;
 }
 
-static cudaError_t launch_update(const UpdParams &u, int rp, bool is_w, cudaStream_t s) {
-    const int grid = ceil_div(u.cols, kUpdCols);
-    const int smem = update_smem_bytes(rp);
+template <int RP>
+static cudaError_t launch_update_rp(const UpdParams &u, cudaLaunchConfig_t &cfg, int rows) {
+    if constexpr (RP <= 64) {
+        return cudaLaunchKernelEx(&cfg, tc_update_kernel<RP, 16>, u);
+    } else {
+        if constexpr (RP <= 128)
+            if (rows == 64) return cudaLaunchKernelEx(&cfg, tc_update_kernel<RP, 64>, u);
+        return cudaLaunchKernelEx(&cfg, tc_update_kernel<RP, 32>, u);
+    }
+}
+
+static cudaError_t launch_update(const UpdParams &u, int rp, cudaStream_t s) {
+    const int rows = upd_rows(u.cols, rp);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kUpdThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3(ceil_div(u.cols, rows));
+    cfg.blockDim = dim3(upd_threads(rp, rows));
+    cfg.dynamicSmemBytes = update_smem_bytes(rp, rows);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -2922,10 +2973,8 @@ static cudaError_t launch_update(const UpdParams &u, int rp, bool is_w, cudaStre
     cfg.attrs = at;
     cfg.numAttrs = 1;
     switch (rp) {
-#define CASE(R)                                                                          \
-    case R:                                                                              \
-        return is_w ? cudaLaunchKernelEx(&cfg, tc_update_kernel<R, true>, u)             \
-                    : cudaLaunchKernelEx(&cfg, tc_update_kernel<R, false>, u);
+#define CASE(R) \
+    case R: return launch_update_rp<R>(u, cfg, rows);
         CASE(16) CASE(32) CASE(48) CASE(64) CASE(80) CASE(96) CASE(112) CASE(128) CASE(144) CASE(160) CASE(176)
         CASE(192)
 #undef CASE
@@ -2937,7 +2986,7 @@ static UpdParams update_params_h(gpunmf_job *j, int update) {
     TcState *t = j->tc;
     UpdParams u{};
     u.X = j->H; u.Xb = t->Hb; u.ldb = t->ldh; u.ldx = 0; u.G = t->G_w; u.P = t->P_h;
-    u.slot_ptr = t->gh.slot_ptr; u.slot_list = t->gh.slot_list; u.tile_slots = t->gh.tile_slots;
+    u.slot_ptr = t->gh.slot_ptr; u.slot_list = t->gh.slot_list;
     u.gram_partials = t->GP_h;
     u.r = j->r; u.cols = j->m; u.npad = t->npad; u.eps = j->eps; u.update = update;
     u.additive = rule_is_additive(j->rule);
@@ -2948,7 +2997,7 @@ static UpdParams update_params_w(gpunmf_job *j, int update) {
     TcState *t = j->tc;
     UpdParams u{};
     u.X = j->W; u.Xb = t->Wb; u.ldb = t->ldw; u.ldx = j->n; u.G = t->G_h; u.P = t->P_w;
-    u.slot_ptr = t->gw.slot_ptr; u.slot_list = t->gw.slot_list; u.tile_slots = t->gw.tile_slots;
+    u.slot_ptr = t->gw.slot_ptr; u.slot_list = t->gw.slot_list; u.is_w = 1;
     u.gram_partials = t->GP_w;
     u.r = j->r; u.cols = j->n; u.npad = t->npad; u.eps = j->eps; u.update = update;
     u.additive = rule_is_additive(j->rule);
@@ -3399,7 +3448,7 @@ size_t tc_footprint(int rule, int n, int m, int r) {
     size_t b = 2 * (2 * (size_t)((n + 127) / 128 * 128) * ((m + 127) / 128 * 128) + (size_t)ceil8(n) * r +
                     (size_t)ceil8(m) * r);
     b += gemm_partial_bytes(m, n, npad) + gemm_partial_bytes(n, m, npad);
-    b += (size_t)npad * npad * sizeof(float) * (2 + ceil_div(n, kUpdCols) + ceil_div(m, kUpdCols)) + 64;
+    b += (size_t)npad * npad * sizeof(float) * (2 + ceil_div(n, kUpdGramRows) + ceil_div(m, kUpdGramRows)) + 64;
     b += fused_bytes(m, npad) + fused_bytes(n, npad);
     return b;
 }
@@ -3426,8 +3475,8 @@ gpunmf_status tc_create(gpunmf_job *j) {
     if (e == cudaSuccess) e = job_dev_alloc(j, (void **)&t->Hb, (size_t)t->ldh * r * 2);
     if (e == cudaSuccess) e = job_dev_alloc(j, (void **)&t->err, sizeof(int));
     const size_t rp2 = (size_t)t->npad * t->npad;
-    t->gp_w_count = ceil_div(n, kUpdCols);
-    t->gp_h_count = ceil_div(m, kUpdCols);
+    t->gp_w_count = ceil_div(n, kUpdGramRows);
+    t->gp_h_count = ceil_div(m, kUpdGramRows);
     if (e == cudaSuccess) e = job_dev_alloc(j, (void **)&t->G_w, rp2 * sizeof(float));
     if (e == cudaSuccess) e = job_dev_alloc(j, (void **)&t->G_h, rp2 * sizeof(float));
     if (e == cudaSuccess) e = job_dev_alloc(j, (void **)&t->GP_w, rp2 * t->gp_w_count * sizeof(float));
@@ -3535,10 +3584,10 @@ gpunmf_status tc_prepare(gpunmf_job *j, const float *v_src) {
         return GPUNMF_OK;
     }
     // Gram partials of the initial W, finished by the first H-step GEMM
-    GPUNMF_CUDA_TRY(launch_update(update_params_w(j, 0), t->npad, true, s));
+    GPUNMF_CUDA_TRY(launch_update(update_params_w(j, 0), t->npad, s));
     // a rule without an H step: the Gram partials of the (fixed) H, finished by every W-step GEMM
     if (j->rule == GPUNMF_ADDITIVE_EUCLIDEAN_FIXED_H)
-        GPUNMF_CUDA_TRY(launch_update(update_params_h(j, 0), t->npad, false, s));
+        GPUNMF_CUDA_TRY(launch_update(update_params_h(j, 0), t->npad, s));
     return GPUNMF_OK;
 }
 
@@ -3624,7 +3673,7 @@ gpunmf_status tc_iterate(gpunmf_job *j, bool updateW) {
         mark_begin(j);
         GPUNMF_CUDA_TRY(launch_gemm(t->gh, s));
         mark_end(j);
-        GPUNMF_CUDA_TRY(launch_update(update_params_h(j, 1), t->npad, false, s));
+        GPUNMF_CUDA_TRY(launch_update(update_params_h(j, 1), t->npad, s));
         j->launches += 2;
     }
     if (!updateW) return GPUNMF_OK;
@@ -3632,7 +3681,7 @@ gpunmf_status tc_iterate(gpunmf_job *j, bool updateW) {
     mark_begin(j);
     GPUNMF_CUDA_TRY(launch_gemm(t->gw, s));
     mark_end(j);
-    GPUNMF_CUDA_TRY(launch_update(update_params_w(j, 1), t->npad, true, s));
+    GPUNMF_CUDA_TRY(launch_update(update_params_w(j, 1), t->npad, s));
     j->launches += 2;
     return GPUNMF_OK;
 }
@@ -3689,7 +3738,7 @@ void tc_destroy(gpunmf_job *j) {
     forget_fused_stream(j->stream);
     void *ptrs[] = {t->Vb, t->Vbt, t->Wb, t->Hb, t->P_h, t->P_w, t->err, t->G_h, t->G_w, t->GP_h, t->GP_w,
                     t->gh.slot_ptr, t->gh.slot_list, t->gw.slot_ptr, t->gw.slot_list,
-                    t->gh.tile_slots, t->gw.tile_slots, t->Wr, t->Hc, t->S_w, t->S_h, t->SP_w, t->SP_h,
+                    t->Wr, t->Hc, t->S_w, t->S_h, t->SP_w, t->SP_h,
                     t->kh.slot_ptr, t->kh.slot_list, t->kh.tile_slots, t->kw.slot_ptr, t->kw.slot_list,
                     t->kh.counters, t->kh.row_sums, t->kw.counters, t->kw.row_sums,
                     t->kw.tile_slots, t->gh.counters, t->gh.grams, t->gw.counters, t->gw.grams};
