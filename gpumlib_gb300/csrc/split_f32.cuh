@@ -59,17 +59,66 @@ struct SpParams {
     double *rout;                // the relative residual
 };
 
-// a - b for two values at once (packed FP32)
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-    unsigned long long d, x, y, m;
-    asm("mov.b64 %0, {%1,%2};" : "=l"(x) : "f"(a.x), "f"(a.y));
-    asm("mov.b64 %0, {%1,%2};" : "=l"(y) : "f"(b.x), "f"(b.y));
-    asm("mov.b64 %0, {%1,%2};" : "=l"(m) : "f"(-1.f), "f"(-1.f));
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(y), "l"(m), "l"(x));
+// packed FP32: two values an operation
+__device__ __forceinline__ unsigned long long bits2(float2 a) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1,%2};" : "=l"(d) : "f"(a.x), "f"(a.y));
+    return d;
+}
+__device__ __forceinline__ float2 vals2(unsigned long long d) {
     float2 r;
     asm("mov.b64 {%0,%1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(d));
     return r;
 }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
+    return vals2(d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)));
+    return vals2(d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)));
+    return vals2(d);
+}
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, both(-1.f), a); }
+
+// log10 of two positive normal values: x = 2^e (1 + f) with sqrt(1/2) <= 1 + f < sqrt(2), and
+// e log10(2) + f Q(f), Q the least-squares polynomial of degree 9 that a reweighted fit (Lawson) takes
+// to the smallest largest relative error, 4e-9.  At most 1.9 units in the last place off over
+// 2^-3 .. 2^3 (log10f promises 2), for a third of log10f's operations.  `range` collects the largest
+// distance of the values' bits from the smallest normal's: below 0x7F000000 all are normal.
+__device__ __forceinline__ float2 log10_pair(float2 x, uint32_t &range) {
+    auto split = [&](float v, float &m) {
+        const int b = __float_as_int(v);
+        range = max(range, (uint32_t)b - 0x00800000u);
+        const int e = (b - 0x3F3504F3) >> 23;
+        m = __int_as_float(b - (e << 23));
+        return __int_as_float(0x4B400000 + e);  // 2^23 * 1.5 + e
+    };
+    float2 m, e;
+    e.x = split(x.x, m.x);
+    e.y = split(x.y, m.y);
+    e = add2(e, both(-12582912.f));
+    const float2 f = add2(m, both(-1.f));
+    float2 q = both(-3.309807181e-02f);
+    q = fma2(q, f, both(5.604422465e-02f));
+    q = fma2(q, f, both(-5.751562491e-02f));
+    q = fma2(q, f, both(6.159092858e-02f));
+    q = fma2(q, f, both(-7.213202864e-02f));
+    q = fma2(q, f, both(8.686744422e-02f));
+    q = fma2(q, f, both(-1.085805073e-01f));
+    q = fma2(q, f, both(1.447647959e-01f));
+    q = fma2(q, f, both(-2.171471864e-01f));
+    q = fma2(q, f, both(4.342944920e-01f));
+    return fma2(e, both(0.30102999566398120f), mul2(q, f));
+}
+
 // cut3 of two finite values, the parts packed: 4.5 operations a value.  (An infinity or NaN
 // becomes NaN in the later parts; the callers see to those.)
 __device__ __forceinline__ void cut_pair(float x0, float x1, uint32_t &w0, uint32_t &w1, uint32_t &w2) {
@@ -92,11 +141,11 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8])
                  : "memory");
 }
 
-// s + c += x with the rounding error of s kept in c (Knuth's TwoSum): a sum as good as one in FP64
-// at the FP32 pipe's rate (this GPU's FP64 pipe would take longer over V than reading it does)
-__device__ __forceinline__ void two_sum(float &s, float &c, float x) {
-    const float t = s + x, bb = t - s;
-    c += (s - (t - bb)) + (x - bb);
+// s + c += x with the rounding error of s kept in c (Knuth's TwoSum), two sums at once: as good as sums
+// in FP64 at the FP32 pipe's rate (this GPU's FP64 pipe would take longer over V than reading it does)
+__device__ __forceinline__ void two_sum(float2 &s, float2 &c, float2 x) {
+    const float2 t = add2(s, x), bb = sub2(t, s);
+    c = add2(c, add2(sub2(s, sub2(t, bb)), sub2(x, bb)));
     s = t;
 }
 
@@ -380,7 +429,8 @@ __global__ void __launch_bounds__(kSpThreads, 1)
         // sixteen workers: a quarter of the rows (their TMEM lanes) by a quarter of the chunk's K for
         // cutting or reducing, by a quarter of the rank for draining.  A chunk is cut while the
         // product of the one before runs, which is drained next.  (V is no kernel's output: without a
-        // first product the first chunk is cut before the wait.)
+        // first product the first chunk is cut before the wait.)  (Two groups of eight that take
+        // chunks in turn, for the reductions, measured the same: their arithmetic bounds them.)
         if constexpr (kFirst) {
             griddep_wait();
             griddep_launch_dependents();
@@ -391,7 +441,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         int vs = 0, rb = 0, d1 = 0, db = 0, kk = kc0, t = t0, seg = 0, dk = kc0, dseg = 0;
         uint32_t vph = 0, rph = 0, d1ph = 0, dph = 0;
-        float qs = 0.f, qc = 0.f, ws = 0.f, wc = 0.f;  // two-term sums
+        float2 qs = both(0.f), qc = qs, ws = qs, wc = qs;  // two-term sums
         float acc[kReduce ? 1 : NC];
         if constexpr (!kReduce) {
 #pragma unroll
@@ -461,6 +511,8 @@ __global__ void __launch_bounds__(kSpThreads, 1)
             }
             if (!mbar_wait(&vfull[vs], vph, p.err, kErrWaitFull, p.wait_limit)) break;
             const uint32_t vt = smem_u32(sVr + vs * kSpVBytes);
+            // K left from this warp's first column (a reduction counts no row beyond the last either)
+            const int klim = kReduce && t * kTileM + row >= p.a1_rows ? 0 : p.kvalid - kk * kSpChunk - part * 16;
             float v[16], s[16];
             if (p.k_contig) {
 #pragma unroll
@@ -472,8 +524,6 @@ __global__ void __launch_bounds__(kSpThreads, 1)
 #pragma unroll
                 for (int c = 0; c < 16; c++) v[c] = lds32_stage(vt + (part * 16 + c) * 512 + row * 4);
             }
-            // K left from this warp's first column (a reduction counts no row beyond the last either)
-            const int klim = kReduce && t * kTileM + row >= p.a1_rows ? 0 : p.kvalid - kk * kSpChunk - part * 16;
             if constexpr (kFirst) {
                 if (!mbar_wait(&d1full[d1], d1ph, p.err, kErrWaitTmemFull, p.wait_limit)) break;
                 tc_fence_after();
@@ -525,15 +575,22 @@ __global__ void __launch_bounds__(kSpThreads, 1)
                     __syncwarp();
                 }
             } else if constexpr (MODE == kSpQuality) {
-                // log10 as log2 times log10(2): both within an ulp of FP32
-                auto term = [&](int c) { return v[c] * (0.30102999566398120f * log2f(s[c] + p.eps)) - s[c]; };
-                if (klim >= 16) {
+                uint32_t range = 0;
+                float2 l[8];
 #pragma unroll
-                    for (int c = 0; c < 16; c++) two_sum(qs, qc, term(c));
-                } else {
+                for (int c = 0; c < 8; c++)
+                    l[c] = log10_pair(add2(make_float2(s[2 * c], s[2 * c + 1]), both(p.eps)), range);
+                if (!__any_sync(0xffffffffu, klim < 16 || range >= 0x7F000000u)) {
+#pragma unroll
+                    for (int c = 0; c < 8; c++) {
+                        const float2 s2 = make_float2(s[2 * c], s[2 * c + 1]);
+                        two_sum(qs, qc, sub2(mul2(make_float2(v[2 * c], v[2 * c + 1]), l[c]), s2));
+                    }
+                } else {  // the edge of V, or a sum that is zero, subnormal, infinite or NaN
 #pragma unroll
                     for (int c = 0; c < 16; c++)
-                        if (c < klim) two_sum(qs, qc, term(c));
+                        if (c < klim)
+                            two_sum(qs, qc, make_float2(v[c] * log10f(s[c] + p.eps) - s[c], 0.f));
                 }
                 __syncwarp();
             } else {
@@ -544,15 +601,15 @@ __global__ void __launch_bounds__(kSpThreads, 1)
                         if (c >= klim) v[c] = s[c] = 0.f;
                 }
 #pragma unroll
-                for (int c = 0; c < 16; c++) {
-                    const float x = v[c], y = s[c];
-                    const float d = x - y, bb = d - x;
-                    const float e = (x - (d - bb)) - (y + bb);
-                    const float dd = d * d, vv = x * x;
+                for (int c = 0; c < 16; c += 2) {
+                    const float2 x = make_float2(v[c], v[c + 1]), y = make_float2(s[c], s[c + 1]);
+                    const float2 d = sub2(x, y), bb = sub2(d, x);
+                    const float2 e = sub2(sub2(x, sub2(d, bb)), add2(y, bb));
+                    const float2 dd = mul2(d, d), vv = mul2(x, x);
                     two_sum(qs, qc, dd);
-                    qc += fmaf(d, d, -dd) + 2.f * d * e;
+                    qc = add2(qc, fma2(add2(d, d), e, fma2(d, d, mul2(dd, both(-1.f)))));
                     two_sum(ws, wc, vv);
-                    wc += fmaf(x, x, -vv);
+                    wc = add2(wc, fma2(x, x, mul2(vv, both(-1.f))));
                 }
             }
             if constexpr (!kReduce) {
@@ -573,6 +630,8 @@ __global__ void __launch_bounds__(kSpThreads, 1)
             // The V stage goes back only here, when what was read of it has been used: given back right
             // after the loads it could be refilled before they were done, where a tcgen05.st held
             // them up (seen at the first chunk of a tile).
+            if constexpr (kReduce)
+                asm volatile("" : "+f"(qs.x), "+f"(qs.y), "+f"(qc.x), "+f"(qc.y), "+f"(ws.x), "+f"(ws.y)::"memory");
             __syncwarp();
             if (lane == 0) {
                 if constexpr (!kReduce) mbar_arrive(&rfull[rb]);
@@ -594,7 +653,8 @@ __global__ void __launch_bounds__(kSpThreads, 1)
             if (j + 1 == nblk) drain(true);
         }
         if constexpr (kReduce) {
-            double a = (double)qs + (double)qc, b = (double)ws + (double)wc;
+            double a = ((double)qs.x + (double)qc.x) + ((double)qs.y + (double)qc.y);
+            double b = ((double)ws.x + (double)wc.x) + ((double)ws.y + (double)wc.y);
             a = warp_sum(a);
             if (MODE == kSpResidual) b = warp_sum(b);
             if (lane == 0) {
