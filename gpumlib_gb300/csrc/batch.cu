@@ -21,6 +21,8 @@
 //
 // Tile shapes (BC, BI) are template parameters; each instance carries the
 // index of the shape an autotuner picked for its (r, size) bucket.
+#include <string.h>
+
 #include <algorithm>
 #include <mutex>
 #include <numeric>
@@ -35,6 +37,7 @@ namespace gpunmf {
 struct BatchInst {
     long long v, w, h;  // offsets (floats) into the packed V, W, H buffers
     int n, m, r, cfg;
+    long long ldv;      // column stride of V
 };
 
 constexpr int kBatchThreads = 256;
@@ -117,7 +120,7 @@ struct InstanceRunner {
     // quality of the current factors, sum V log10(WH + eps) - WH (nmf_kernels_quality.cu:35), as the
     // float the reference reads back; WH is formed tile by tile and never stored.  Same value on
     // every thread.  Uses the V, factor and chunk areas of shared memory, not the Gram.
-    __device__ __noinline__ static float quality(const float *__restrict__ V, const float *__restrict__ W,
+    __device__ __noinline__ static float quality(const float *__restrict__ V, long long ldv, const float *__restrict__ W,
                                     const float *__restrict__ H, int n, int m, int r, float eps, float *sm) {
         __shared__ double qred[32];
         float *sV = sm + OFF_V, *sF = sm + OFF_F, *sX = sm + OFF_X;
@@ -137,7 +140,7 @@ struct InstanceRunner {
                 for (int k = tid; k < BI * BC; k += kBatchThreads) {
                     const int u = k / BI, ii = k % BI;
                     const bool ok = ii < nr && u < nc;
-                    cp_async_f32(&sV[ii * (BC + 4) + u], ok ? V + (long long)(c0 + u) * n + i0 + ii : V, ok);
+                    cp_async_f32(&sV[ii * (BC + 4) + u], ok ? V + (c0 + u) * ldv + i0 + ii : V, ok);
                 }
                 for (int k = tid; k < BI * R; k += kBatchThreads) {
                     const int a = k / BI, ii = k % BI;
@@ -169,6 +172,7 @@ struct InstanceRunner {
                                float *__restrict__ Hall, float eps, int iters, float *sm,
                                const BatchStop &stop, int inst) {
         const int n = d.n, m = d.m, r = d.r;
+        const long long ldv = d.ldv;
         const float *V = Vall + d.v;
         float *W = Wall + d.w;
         float *H = Hall + d.h;
@@ -190,7 +194,7 @@ struct InstanceRunner {
         int done = iters;
         for (int it = 0; it < iters; it++) {
             if constexpr (kStop) {
-                const float q_new = quality(V, W, H, n, m, r, eps, sm);  // contains barriers
+                const float q_new = quality(V, d.ldv, W, H, n, m, r, eps, sm);  // contains barriers
                 if (tid == 0) {
                     const float q_now = lag.value;
                     if (lag.times++ > 2) lag.delta = q_now - lag.last;
@@ -221,7 +225,7 @@ struct InstanceRunner {
                     for (int k = tid; k < BI * BC; k += kBatchThreads) {
                         const int u = k / BI, ii = k % BI;
                         const bool ok = ii < nr && u < nc;
-                        cp_async_f32(&sV[ii * (BC + 4) + u], ok ? V + (long long)(c0 + u) * n + i0 + ii : V, ok);
+                        cp_async_f32(&sV[ii * (BC + 4) + u], ok ? V + (c0 + u) * ldv + i0 + ii : V, ok);
                     }
                     for (int k = tid; k < BI * R; k += kBatchThreads) {
                         const int a = k / BI, ii = k % BI;
@@ -309,7 +313,7 @@ struct InstanceRunner {
                     for (int k = tid; k < BI * BC; k += kBatchThreads) {
                         const int uu = k / BC, ii = k % BC;
                         const bool ok = ii < nr && uu < ncu;
-                        cp_async_f32(&sV[uu * (BC + 4) + ii], ok ? V + (long long)(u0 + uu) * n + i0 + ii : V, ok);
+                        cp_async_f32(&sV[uu * (BC + 4) + ii], ok ? V + (u0 + uu) * ldv + i0 + ii : V, ok);
                     }
                     for (int k = tid; k < BI * R; k += kBatchThreads) {
                         const int uu = k / R, a = k % R;
@@ -444,7 +448,7 @@ __global__ void batch_residual_kernel(const BatchInst *__restrict__ insts, int c
         const int i = (int)(e % d.n), u = (int)(e / d.n);
         float wh = 0.f;
         for (int a = 0; a < d.r; a++) wh = fmaf(w[(long long)a * d.n + i], h[(long long)u * d.r + a], wh);
-        const double x = v[e], dd = x - (double)wh;
+        const double x = v[u * d.ldv + i], dd = x - (double)wh;
         num += dd * dd;
         den += x * x;
     }
@@ -474,6 +478,8 @@ struct gpunmf_batch {
     cudaGraphExec_t graph = nullptr;
     int graph_iters = -1;
     int grid = 0;
+    unsigned char *h_pinned = nullptr;  // page-locked room for the largest instance's W and H (gpunmf_batch_get)
+    SpBatch *split = nullptr;  // the half-steps of all instances share their launches (split_batch.cuh)
 };
 
 static int rank_class(int r) { return r <= 4 ? 4 : r <= 8 ? 8 : r <= 16 ? 16 : r <= 32 ? 32 : 0; }
@@ -519,6 +525,8 @@ static void order_largest_first(const std::vector<BatchInst> &in, std::vector<in
 static void batch_free(gpunmf_batch *b) {
     if (!b) return;
     if (b->graph) cudaGraphExecDestroy(b->graph);
+    spb_destroy(b->split);
+    if (b->h_pinned) cudaFreeHost(b->h_pinned);
     void *ptrs[] = {b->d_insts, b->d_order, b->d_next, b->V, b->W, b->H, b->d_res};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -575,7 +583,8 @@ gpunmf_status gpunmf_batch_create(int count, const int *n, const int *m, const i
         BatchInst &d = b->h_insts[k];
         d.n = n[k]; d.m = m[k]; d.r = r[k]; d.cfg = default_cfg(r[k]);
         d.v = b->v_total; d.w = b->w_total; d.h = b->h_total;
-        b->v_total += ((long long)n[k] * m[k] + 3) / 4 * 4;
+        d.ldv = (n[k] + 3) / 4 * 4;
+        b->v_total += d.ldv * m[k];
         b->w_total += ((long long)n[k] * r[k] + 3) / 4 * 4;
         b->h_total += ((long long)r[k] * m[k] + 3) / 4 * 4;
     }
@@ -610,7 +619,10 @@ gpunmf_status gpunmf_batch_create(int count, const int *n, const int *m, const i
             const float *src = kind == 0 ? V[k] : kind == 1 ? W[k] : H[k];
             long long off = kind == 0 ? d.v : kind == 1 ? d.w : d.h;
             long long cnt = kind == 0 ? (long long)d.n * d.m : kind == 1 ? (long long)d.n * d.r : (long long)d.r * d.m;
-            std::copy(src, src + cnt, stage + off);
+            if (kind == 0 && d.ldv != d.n)
+                for (int u = 0; u < d.m; u++) std::copy(src + (long long)u * d.n, src + (long long)(u + 1) * d.n, stage + off + u * d.ldv);
+            else
+                std::copy(src, src + cnt, stage + off);
         }
         float *dst = kind == 0 ? b->V : kind == 1 ? b->W : b->H;
         cudaError_t ce = cudaMemcpyAsync(dst, stage, sizeof(float) * total, cudaMemcpyHostToDevice, b->stream);
@@ -622,12 +634,30 @@ gpunmf_status gpunmf_batch_create(int count, const int *n, const int *m, const i
             return GPUNMF_ERR_CUDA;
         }
     }
+    size_t largest = 0;
+    for (const BatchInst &d : b->h_insts) largest = std::max(largest, sizeof(float) * (size_t)d.r * ((size_t)d.n + d.m));
+    if (cudaHostAlloc((void **)&b->h_pinned, largest, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();  // without it the copies go straight to the caller's memory
+        b->h_pinned = nullptr;
+    }
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<false>, kBatchThreads, batch_max_smem());
     b->grid = std::max(1, sms * std::max(1, per_sm));
     gpunmf_status st = batch_upload_order(b);
+    if (st == GPUNMF_OK) {
+        std::vector<SpbShape> shapes(count);
+        for (int k = 0; k < count; k++) {
+            const BatchInst &d = b->h_insts[k];
+            shapes[k] = SpbShape{d.n, d.m, d.r, b->V + d.v, b->W + d.w, b->H + d.h};
+        }
+        if (spb_better(shapes)) {
+            st = spb_create(shapes, eps, b->stream, &b->split);
+            if (st == GPUNMF_OK) st = spb_reset(b->split, b->stream);
+            else if (st == GPUNMF_ERR_NOMEM) st = GPUNMF_OK;  // the one-CTA kernel needs no more memory
+        }
+    }
     if (st != GPUNMF_OK) {
         batch_free(b);
         return st;
@@ -648,6 +678,7 @@ gpunmf_status gpunmf_batch_destroy(gpunmf_batch *b) {
 gpunmf_status gpunmf_batch_run(gpunmf_batch *b, int iters) {
     if (!b || iters < 0) return GPUNMF_ERR_INVALID;
     if (iters == 0) return GPUNMF_OK;
+    if (b->split) return spb_run(b->split, iters, b->stream);
     if (!b->graph || b->graph_iters != iters) {
         if (b->graph) {
             cudaGraphExecDestroy(b->graph);
@@ -675,7 +706,7 @@ gpunmf_status gpunmf_batch_run(gpunmf_batch *b, int iters) {
 gpunmf_status gpunmf_batch_synchronize(gpunmf_batch *b) {
     if (!b) return GPUNMF_ERR_INVALID;
     GPUNMF_CUDA_TRY(cudaStreamSynchronize(b->stream));
-    return GPUNMF_OK;
+    return b->split ? spb_check(b->split, b->stream) : GPUNMF_OK;
 }
 
 // Device time of `iters` iterations of the whole batch (one graph launch), in ms.
@@ -701,9 +732,19 @@ gpunmf_status gpunmf_batch_time(gpunmf_batch *b, int iters, float *ms) {
 gpunmf_status gpunmf_batch_get(gpunmf_batch *b, int k, float *W, float *H) {
     if (!b || k < 0 || k >= b->count) return GPUNMF_ERR_INVALID;
     const BatchInst &d = b->h_insts[k];
-    if (W) GPUNMF_CUDA_TRY(cudaMemcpyAsync(W, b->W + d.w, sizeof(float) * (size_t)d.n * d.r, cudaMemcpyDeviceToHost, b->stream));
-    if (H) GPUNMF_CUDA_TRY(cudaMemcpyAsync(H, b->H + d.h, sizeof(float) * (size_t)d.r * d.m, cudaMemcpyDeviceToHost, b->stream));
+    const size_t wb = sizeof(float) * (size_t)d.n * d.r, hb = sizeof(float) * (size_t)d.r * d.m;
+    // through page-locked memory: both copies are in flight at once and one wait ends them (to pageable
+    // memory each copy waits for itself: 33 us a call against 12)
+    float *pw = W, *ph = H;
+    if (b->h_pinned) {
+        pw = reinterpret_cast<float *>(b->h_pinned);
+        ph = pw + (size_t)d.n * d.r;
+    }
+    if (W) GPUNMF_CUDA_TRY(cudaMemcpyAsync(pw, b->W + d.w, wb, cudaMemcpyDeviceToHost, b->stream));
+    if (H) GPUNMF_CUDA_TRY(cudaMemcpyAsync(ph, b->H + d.h, hb, cudaMemcpyDeviceToHost, b->stream));
     GPUNMF_CUDA_TRY(cudaStreamSynchronize(b->stream));
+    if (W && pw != W) memcpy(W, pw, wb);
+    if (H && ph != H) memcpy(H, ph, hb);
     return GPUNMF_OK;
 }
 
@@ -753,6 +794,10 @@ gpunmf_status gpunmf_batch_reset_factors(gpunmf_batch *b, const float *const *W,
         const BatchInst &d = b->h_insts[k];
         GPUNMF_CUDA_TRY(cudaMemcpyAsync(b->W + d.w, W[k], sizeof(float) * (size_t)d.n * d.r, cudaMemcpyHostToDevice, b->stream));
         GPUNMF_CUDA_TRY(cudaMemcpyAsync(b->H + d.h, H[k], sizeof(float) * (size_t)d.r * d.m, cudaMemcpyHostToDevice, b->stream));
+    }
+    if (b->split) {
+        gpunmf_status st = spb_reset(b->split, b->stream);
+        if (st != GPUNMF_OK) return st;
     }
     GPUNMF_CUDA_TRY(cudaStreamSynchronize(b->stream));
     return GPUNMF_OK;
@@ -930,7 +975,7 @@ extern "C" gpunmf_status gpunmf_grouped_train(int rule, int n, int m, int r, int
         std::vector<int> order(blocks);
         for (int b = 0; b < blocks; b++) {
             BatchInst &d = insts[b];
-            d.n = n; d.m = group; d.r = rs; d.cfg = default_cfg(rs);
+            d.n = n; d.m = group; d.r = rs; d.cfg = default_cfg(rs); d.ldv = n;
             d.v = (long long)b * n * group;
             d.w = (long long)b * n * rs;
             d.h = (long long)b * rs * group;

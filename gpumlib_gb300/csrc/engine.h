@@ -8,6 +8,7 @@
 #include "../../include/gpunmf.h"
 
 struct TcState;  // tensor-core path state (tc_kernels.cu)
+struct SpBatch;  // batches on the tensor cores (split_batch.cuh)
 struct SpState;  // FP32 products on the tensor cores (split_f32.cuh)
 
 struct gpunmf_job {
@@ -118,6 +119,18 @@ bool sp_quality_writes_host(const gpunmf_job *j);
 gpunmf_status sp_residual(gpunmf_job *j, double *d_out);
 void sp_destroy(gpunmf_job *j);
 void job_residual_ready(gpunmf_job *j);  // before the first job_residual (may allocate)
+// batches of Euclidean instances of rank <= 32 by the FP32 products (split_batch.cuh)
+struct SpbShape {
+    int n, m, r;
+    const float *V;  // device, column stride n rounded up to 4
+    float *W, *H;
+};
+bool spb_better(const std::vector<SpbShape> &shapes);
+gpunmf_status spb_create(const std::vector<SpbShape> &shapes, float eps, cudaStream_t s, SpBatch **out);
+gpunmf_status spb_reset(SpBatch *b, cudaStream_t s);
+gpunmf_status spb_run(SpBatch *b, int iters, cudaStream_t s);
+gpunmf_status spb_check(SpBatch *b, cudaStream_t s);
+void spb_destroy(SpBatch *b);
 // the job's relative residual, enqueued on its stream, into *d_out
 gpunmf_status job_residual(gpunmf_job *j, double *d_out);
 }  // namespace gpunmf

@@ -725,6 +725,13 @@ __global__ void sp_cut_factors_kernel(const float *__restrict__ W, int n, const 
     }
 }
 
+// V (n x m) with its columns ld apart
+__global__ void sp_pad_columns_kernel(const float *__restrict__ V, int n, int m, float *__restrict__ out, long long ld) {
+    for (long long u = blockIdx.y; u < m; u += gridDim.y)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+            out[u * ld + i] = V[u * n + i];
+}
+
 // ------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------
@@ -1060,7 +1067,7 @@ static cudaError_t sp_update(gpunmf_job *j, bool is_w, int update) {
     u.gram_partials = is_w ? t->GP_w : t->GP_h;
     u.r = j->r; u.cols = rows; u.npad = t->npad; u.eps = j->eps; u.update = update;
     u.additive = rule_is_additive(j->rule);
-    u.V = j->V; u.F = is_w ? j->H : j->W; u.K = is_w ? j->m : j->n;
+    u.V = j->V; u.ldv = j->n; u.F = is_w ? j->H : j->W; u.K = is_w ? j->m : j->n;
     return launch_update(u, t->npad, j->stream);
 }
 
@@ -1075,9 +1082,9 @@ static cudaError_t sp_cut_factors(gpunmf_job *j) {
 gpunmf_status sp_prepare(gpunmf_job *j, bool residual_only) {
     SpState *t = j->sp;
     if (t->Vp) {
-        const size_t ldv = (size_t)(j->n + 3) / 4 * 4;
-        GPUNMF_CUDA_TRY(cudaMemcpy2DAsync(t->Vp, ldv * 4, j->V, (size_t)j->n * 4, (size_t)j->n * 4, j->m,
-                                          cudaMemcpyDeviceToDevice, j->stream));
+        sp_pad_columns_kernel<<<dim3(std::min(ceil_div(j->n, 256), 8), std::min(j->m, 65535)), 256, 0, j->stream>>>(
+            j->V, j->n, j->m, t->Vp, (j->n + 3) / 4 * 4);
+        GPUNMF_CUDA_TRY(cudaGetLastError());
     }
     if (residual_only) return GPUNMF_OK;
     GPUNMF_CUDA_TRY(sp_cut_factors(j));

@@ -155,12 +155,15 @@ struct FusedLayout {
 
 __device__ __forceinline__ void wk_bar() { asm volatile("bar.sync 2, 64;" ::: "memory"); }
 
-// N consecutive floats from shared memory, N * 4-byte aligned (N = 4: one 16-byte load)
+// N consecutive floats from shared memory, N * 4-byte aligned (16-byte loads where N is a multiple of 4)
 template <int N>
 __device__ __forceinline__ void lds_vec(const float *src, float (&v)[N]) {
-    if constexpr (N == 4) {
-        const float4 t = *reinterpret_cast<const float4 *>(src);
-        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4) {
+            const float4 t = *reinterpret_cast<const float4 *>(src + i);
+            v[i] = t.x; v[i + 1] = t.y; v[i + 2] = t.z; v[i + 3] = t.w;
+        }
     } else if constexpr (N == 2) {
         const float2 t = *reinterpret_cast<const float2 *>(src);
         v[0] = t.x; v[1] = t.y;
@@ -1556,7 +1559,7 @@ struct UpdParams {
     long long ldb;
     long long ldx;            // n for W (W(c,a) at a*n + c); unused for H (H(a,c) at c*r + a)
     const float *G;           // r x r Gram for the denominator
-    const float *P;           // GEMM partial slots [slot][128][npad]
+    const float *P;           // GEMM partial slots [slot][128][RP], npad * 128 floats apart
     const int *slot_ptr, *slot_list;
     float *gram_partials;     // [partial][RP*RP]
     int r, cols, npad;
@@ -1566,17 +1569,19 @@ struct UpdParams {
     int additive;             // 1: X = max(0, X + (X / den) (num - den)) (nmf_kernels.cu:31-38)
     __nv_bfloat16 *Xs;        // FP32 products: the three parts of X instead of Xb, at part * q + c * RP + a
     long long part;
-    const float *V, *F;       // FP32 products: V (column-major) and the other factor, for plain_sum
+    const float *V, *F;       // FP32 products: V (column-major, stride ldv) and the other factor, for plain_sum
+    long long ldv;
     int K;
+    int slot0, slots;         // batches (slot_ptr null): the tile's slots, numbered on
 };
 
 // A numerator of the FP32 products by plain FP32 fused multiply-adds, where the sum of the parts'
 // products is not finite: a part of an infinity or NaN has lost which of the two it was.
-__device__ __noinline__ float plain_sum(const UpdParams &p, int row, int a) {
+__device__ __noinline__ float plain_sum(int is_w, const float *V, long long ldv, const float *F, int r, int K, int row, int a) {
     float s = 0.f;
-    for (int k = 0; k < p.K; k++)
-        s = p.is_w ? fmaf(p.V[(long long)k * p.cols + row], p.F[(long long)k * p.r + a], s)
-                 : fmaf(p.V[(long long)row * p.K + k], p.F[(long long)a * p.K + k], s);
+    for (int k = 0; k < K; k++)
+        s = is_w ? fmaf(V[(long long)k * ldv + row], F[(long long)k * r + a], s)
+                 : fmaf(V[(long long)row * ldv + k], F[(long long)a * K + k], s);
     return s;
 }
 
@@ -1610,21 +1615,18 @@ __device__ __forceinline__ void upd_lds(const float *row, int g, float (&v)[TA])
     for (int i = 0; i < TA; i += V) lds_vec<V>(row + upd_col<TA>(g, i), *reinterpret_cast<float (*)[V]>(&v[i]));
 }
 
-template <int RP, int ROWS>
-__global__ void __launch_bounds__(upd_threads(RP, ROWS)) tc_update_kernel(UpdParams p) {
-    constexpr int NT = upd_threads(RP, ROWS);
+// rows c0 .. c0 + ROWS - 1 of the factor, by NT threads; part: the index of their Gram partial (BF16 jobs:
+// of the first 16 rows'), sm: update_smem_bytes
+template <int RP, int ROWS, int NT>
+__device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part, float *sm) {
     constexpr int TA = RP / 16, RT = ROWS * 16 / NT;
     constexpr int LDX = ROWS + 4, LDN = RP + 4;
-    extern __shared__ __align__(16) float sm[];
     float *Gs = sm;               // [RP][RP], zero outside r
     float *Xs = Gs + RP * RP;     // [RP][LDX]  the old X(a, row)
     float *Ns = Xs + RP * LDX;    // [ROWS][LDN]  numerators, then the new X
     const int tid = threadIdx.x;
-    const int c0 = blockIdx.x * ROWS;
     const int ncol = min(ROWS, p.cols - c0);
     const int r = p.r;
-    griddep_wait();  // the GEMM's partial slots and Gram are complete
-    griddep_launch_dependents();
     // the old rows, zero outside r and ncol; a thread issues up to sixteen loads before it stores
     constexpr int XL = RP * ROWS / NT, XB = XL < 16 ? XL : 16;
 #pragma unroll 1
@@ -1661,7 +1663,7 @@ __global__ void __launch_bounds__(upd_threads(RP, ROWS)) tc_update_kernel(UpdPar
         // numerators: the tile's slots summed in their order, four slots' loads of a thread together.
         // (Rows of a slot beyond the last are in bounds, the tile has 128; they are never stored.)
         const int tile = c0 / 128, lrow0 = c0 % 128;
-        const int s0 = p.slot_ptr[tile], s1 = p.slot_ptr[tile + 1];
+        const int s0 = p.slot_ptr ? p.slot_ptr[tile] : p.slot0, s1 = p.slot_ptr ? p.slot_ptr[tile + 1] : p.slot0 + p.slots;
         constexpr int N4 = ROWS * RP / 4;
 #pragma unroll 1
         for (int k0 = 0; k0 < N4; k0 += 2 * NT) {
@@ -1674,8 +1676,8 @@ __global__ void __launch_bounds__(upd_threads(RP, ROWS)) tc_update_kernel(UpdPar
                 float4 va[4], vb[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const int slot = p.slot_list[min(q0 + q, s1 - 1)];
-                    const float4 *src = reinterpret_cast<const float4 *>(p.P + ((size_t)slot * 128 + lrow0) * RP);
+                    const int sq = min(q0 + q, s1 - 1), slot = p.slot_ptr ? p.slot_list[sq] : sq;
+                    const float4 *src = reinterpret_cast<const float4 *>(p.P + (size_t)slot * 128 * p.npad + lrow0 * RP);
                     if (oa) va[q] = __ldcg(src + ka);
                     if (ob) vb[q] = __ldcg(src + kb);
                 }
@@ -1690,10 +1692,11 @@ __global__ void __launch_bounds__(upd_threads(RP, ROWS)) tc_update_kernel(UpdPar
                 const int c = k / (RP / 4), a = (k % (RP / 4)) * 4;
                 const float inf = __int_as_float(0x7F800000);
                 if (p.Xs && c < ncol && !(fabsf(v.x) < inf && fabsf(v.y) < inf && fabsf(v.z) < inf && fabsf(v.w) < inf)) {
-                    if (!(fabsf(v.x) < inf) && a < r) v.x = plain_sum(p, c0 + c, a);
-                    if (!(fabsf(v.y) < inf) && a + 1 < r) v.y = plain_sum(p, c0 + c, a + 1);
-                    if (!(fabsf(v.z) < inf) && a + 2 < r) v.z = plain_sum(p, c0 + c, a + 2);
-                    if (!(fabsf(v.w) < inf) && a + 3 < r) v.w = plain_sum(p, c0 + c, a + 3);
+                    auto sum = [&](int aa) { return plain_sum(p.is_w, p.V, p.ldv, p.F, r, p.K, c0 + c, aa); };
+                    if (!(fabsf(v.x) < inf) && a < r) v.x = sum(a);
+                    if (!(fabsf(v.y) < inf) && a + 1 < r) v.y = sum(a + 1);
+                    if (!(fabsf(v.z) < inf) && a + 2 < r) v.z = sum(a + 2);
+                    if (!(fabsf(v.w) < inf) && a + 3 < r) v.w = sum(a + 3);
                 }
                 *reinterpret_cast<float4 *>(Ns + c * LDN + a) = v;
             };
@@ -1808,15 +1811,14 @@ __global__ void __launch_bounds__(upd_threads(RP, ROWS)) tc_update_kernel(UpdPar
                         for (int k = 0; k < TA; k++) Gs[(i * TA + k) * 256 + (tid & 255)] = acc[i][k];
                 }
                 __syncthreads();
-                if (half == 1) return;
+                if (half == 1) break;
 #pragma unroll
                 for (int i = 0; i < TA; i++)
 #pragma unroll
                     for (int k = 0; k < TA; k++) acc[i][k] += Gs[(i * TA + k) * 256 + tid];
             }
-            const int part = p.Xs ? blockIdx.x : blockIdx.x * (ROWS / 16) + c1 / 16;
             if (p.Xs || c1 < ncol) {
-                float *out = p.gram_partials + (size_t)part * RP * RP;
+                float *out = p.gram_partials + (size_t)(p.Xs ? part : part + c1 / 16) * RP * RP;
 #pragma unroll
                 for (int i = 0; i < TA; i++)
 #pragma unroll
@@ -1824,6 +1826,14 @@ __global__ void __launch_bounds__(upd_threads(RP, ROWS)) tc_update_kernel(UpdPar
             }
         }
     }
+}
+
+template <int RP, int ROWS>
+__global__ void __launch_bounds__(upd_threads(RP, ROWS)) tc_update_kernel(UpdParams p) {
+    extern __shared__ __align__(16) float sm[];
+    griddep_wait();  // the GEMM's partial slots and Gram are complete
+    griddep_launch_dependents();
+    update_rows<RP, ROWS, upd_threads(RP, ROWS)>(p, blockIdx.x * ROWS, blockIdx.x * (p.Xs ? 1 : ROWS / kUpdGramRows), sm);
 }
 
 // ------------------------------------------------------------------------
@@ -3263,6 +3273,7 @@ static KlUpdParams kl_params_w(gpunmf_job *j, int update) {
 }
 
 #include "split_f32.cuh"
+#include "split_batch.cuh"
 
 static gpunmf_status setup_quality(gpunmf_job *j);
 
