@@ -703,10 +703,12 @@ __global__ void __launch_bounds__(64) gram_partials_kernel(const float *__restri
         if (gb0 + k <= ga) out[(size_t)c * tri_stride(NP) + ga * (ga + 1) / 2 + gb0 + k] = gacc[k];
 }
 
-// threads of the GEMM: producer, MMA issuer, four TMEM-draining warps, with a fused update two
-// worker warps, and with a folded quality sample eight quality warps (warps 8-15)
+// threads of the GEMM: producer, MMA issuer, four TMEM-draining warps; without a fused update ten warps
+// that finish the Gram, else two worker warps, and with a folded quality sample eight quality warps
+// (warps 8-15)
+constexpr int kGramWarps = 10;
 __host__ __device__ constexpr int gemm_threads(int fnp, bool qf = false) {
-    return (fnp ? kGemmThreads + 64 : kGemmThreads) + (qf ? 256 : 0);
+    return kGemmThreads + (fnp ? 64 : 32 * kGramWarps) + (qf ? 256 : 0);
 }
 constexpr int kQfWarps = 8;
 constexpr uint32_t kQfTmemS = 128;  // TMEM column of the first of the 128-column S buffers
@@ -790,7 +792,7 @@ __global__ void __launch_bounds__(gemm_threads(FNP, QF), 1)
     if (FNP == 0 && (int)blockIdx.x >= ctas) {  // no blocks of the product: a share of the Gram only
         griddep_wait();
         griddep_launch_dependents();
-        if (p.gram_out) finish_gram(p, threadIdx.x, kGemmThreads);
+        if (p.gram_out) finish_gram(p, threadIdx.x, gemm_threads(0));
         return;
     }
     const long long T = (long long)p.tiles * p.kblocks;
@@ -994,9 +996,6 @@ __global__ void __launch_bounds__(gemm_threads(FNP, QF), 1)
     } else if (warp < 6) {
         griddep_wait();
         griddep_launch_dependents();
-        // while the first accumulator fills, finish this CTA's share of the Gram matrix that the update
-        // kernel of the previous half-step left as partials
-        if (FNP == 0 && p.gram_out) finish_gram(p, threadIdx.x - 64, 128);
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         int acc = 0, seg = 0;
@@ -1039,7 +1038,14 @@ __global__ void __launch_bounds__(gemm_threads(FNP, QF), 1)
             seg++;
             b = e;
         }
-    } else if constexpr (FNP > 0) {
+    } else if constexpr (FNP == 0) {
+        // this CTA's share of the Gram matrix that the update kernel of the previous half-step left as
+        // partials (by the four draining warps it took longer than the product: 500 x 500, r = 100, 55.8 us
+        // an iteration against 44.8)
+        griddep_wait();
+        griddep_launch_dependents();
+        if (p.gram_out) finish_gram(p, threadIdx.x - kGemmThreads, 32 * kGramWarps);
+    } else {
       if (warp < 8) {
         griddep_wait();
         griddep_launch_dependents();
@@ -1587,18 +1593,13 @@ __device__ __noinline__ float plain_sum(int is_w, const float *V, long long ldv,
 
 // Rows per CTA and its threads.  Up to rank 64: 16 rows, 256 threads; several CTAs of an SM overlap their
 // latencies (8192 x 8192, r = 64, an iteration: 16 rows 131 us, 32 132, 64 152).  Above, every CTA's
-// r x r matrices weigh more: 64 rows and 512 threads where that still makes about one CTA for every
-// other SM (r = 128, an iteration: 8192 rows 64 / 32 / 16 193 / 224 / 307 us, 4000 rows 108 / 100; the
-// factors' odd multiples of 16, read one value at a time: 3000 rows of r = 80 62 / 65), else 32 rows
-// with 512 threads, or 256 for the odd multiples (500 rows, r = 100: 55 us against 74).  Above rank
-// 128 G leaves room for 32 rows only.
-__host__ __device__ constexpr bool upd_odd(int rp) { return rp / 16 % 2 != 0; }
+// r x r matrices weigh more: 512 threads and 32 rows, or 64 where 32 make more than an SM's worth of CTAs
+// (an iteration in FP32, r = 128: 8192 rows 196 us with 64, 228 with 32; 3000 rows 102 and 94; BF16
+// r = 100: 500 rows 60 and 45).  Above rank 128 G leaves room for 32 rows only.
 __host__ __device__ constexpr int upd_rows(int rows, int rp) {
-    return rp <= 64 ? 16 : rp <= 128 && rows > (upd_odd(rp) ? 2048 : 32 * kNumSMsGB300) ? 64 : 32;
+    return rp <= 64 ? 16 : rp <= 128 && rows > 32 * kNumSMsGB300 ? 64 : 32;
 }
-__host__ __device__ constexpr int upd_threads(int rp, int cta_rows) {
-    return rp > 64 && rp <= 128 && (cta_rows == 64 || !upd_odd(rp)) ? 512 : 256;
-}
+__host__ __device__ constexpr int upd_threads(int rp) { return rp > 64 && rp <= 128 ? 512 : 256; }
 
 // A thread's columns of the rank: vectors of four (or two) 16 vectors apart, so that the 16 threads of a
 // row read neighbouring vectors
@@ -1829,11 +1830,11 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
 }
 
 template <int RP, int ROWS>
-__global__ void __launch_bounds__(upd_threads(RP, ROWS)) tc_update_kernel(UpdParams p) {
+__global__ void __launch_bounds__(upd_threads(RP)) tc_update_kernel(UpdParams p) {
     extern __shared__ __align__(16) float sm[];
     griddep_wait();  // the GEMM's partial slots and Gram are complete
     griddep_launch_dependents();
-    update_rows<RP, ROWS, upd_threads(RP, ROWS)>(p, blockIdx.x * ROWS, blockIdx.x * (p.Xs ? 1 : ROWS / kUpdGramRows), sm);
+    update_rows<RP, ROWS, upd_threads(RP)>(p, blockIdx.x * ROWS, blockIdx.x * (p.Xs ? 1 : ROWS / kUpdGramRows), sm);
 }
 
 // ------------------------------------------------------------------------
@@ -2823,7 +2824,7 @@ static gpunmf_status setup_gemm(gpunmf_job *j, TcGemm &g, int rows, int K, int n
     // Where the product makes few CTAs, more of them share the Gram's npad^2 entries: 500 x 500, r = 100,
     // took 22.7 us a launch with the product's 16 CTAs alone (the Gram 15 of them).
     g.p.ctas = g.grid;
-    if (!fnp) g.grid = std::max(g.grid, std::min(j->tc->max_ctas, npad * npad / (kGemmThreads / 4)));
+    if (!fnp) g.grid = std::max(g.grid, std::min(j->tc->max_ctas, npad * npad / (gemm_threads(0) / 4)));
     g.smem = 1024 + stages * stage_bytes + (2 * stages + 5) * 8 + 16 + (fnp ? 16 + fused_smem_bytes(fnp) : 0);
     // with the folded quality sample: two H-tile slots, eight more barriers, the warps' sums
     g.smem_qf = g.smem + 2 * 2 * npad * kBlockK * 2 + (4 + 2 * kQfSBufs) * 8 + 2 * kQfWarps * 8;
@@ -2974,7 +2975,7 @@ static cudaError_t launch_update(const UpdParams &u, int rp, cudaStream_t s) {
     const int rows = upd_rows(u.cols, rp);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ceil_div(u.cols, rows));
-    cfg.blockDim = dim3(upd_threads(rp, rows));
+    cfg.blockDim = dim3(upd_threads(rp));
     cfg.dynamicSmemBytes = update_smem_bytes(rp, rows);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
