@@ -347,8 +347,6 @@ __global__ void __launch_bounds__(kSpbUpdThreads, 4) spb_update_kernel(SpbUpdPar
     u.V = d.V;
     u.ldv = d.ldv;
     u.F = p.is_w ? d.H : d.W;
-    griddep_wait();
-    griddep_launch_dependents();
     if (d.npad == 16) update_rows<16, kSpbRows, kSpbUpdThreads>(u, b.row0, b.row0 / kSpbRows, sm);
     else update_rows<32, kSpbRows, kSpbUpdThreads>(u, b.row0, b.row0 / kSpbRows, sm);
 }

@@ -703,13 +703,18 @@ __global__ void __launch_bounds__(64) gram_partials_kernel(const float *__restri
         if (gb0 + k <= ga) out[(size_t)c * tri_stride(NP) + ga * (ga + 1) / 2 + gb0 + k] = gacc[k];
 }
 
-// threads of the GEMM: producer, MMA issuer, four TMEM-draining warps; without a fused update ten warps
-// that finish the Gram, else two worker warps, and with a folded quality sample eight quality warps
-// (warps 8-15)
-constexpr int kGramWarps = 10;
-__host__ __device__ constexpr int gemm_threads(int fnp, bool qf = false) {
-    return kGemmThreads + (fnp ? 64 : 32 * kGramWarps) + (qf ? 256 : 0);
+// threads of the GEMM: producer, MMA issuer, four TMEM-draining warps; without a fused update the warps
+// that finish the Gram (gram_threads), else two worker warps, and with a folded quality sample eight
+// quality warps (warps 8-15)
+__host__ __device__ constexpr int gemm_threads(int fnp, bool qf, int gram) {
+    return kGemmThreads + (fnp ? 64 : gram) + (qf ? 256 : 0);
 }
+// Ten warps, four where the Gram is small, two where it is smaller still and the product's CTAs many:
+// the registers they leave let CTAs of the update kernel start beside them (4000 x 5000, r = 10, an
+// iteration with ten / four / two: 27.1 / 24.4 / 23.8 us; 200 x 300, r = 10, four / two 12.1 / 13.5; 500 x 500,
+// r = 100, with the four draining warps instead 55.8, with ten 44.8).
+constexpr int kMaxGramThreads = 320;
+static int gram_threads(int npad, int ctas) { return npad <= 16 && ctas > kNumSMsGB300 / 2 ? 64 : npad <= 48 ? 128 : kMaxGramThreads; }
 constexpr int kQfWarps = 8;
 constexpr uint32_t kQfTmemS = 128;  // TMEM column of the first of the 128-column S buffers
 // S buffers (TMEM, 128 columns each, after the two accumulators): three, so that the MMA of a block's S
@@ -761,7 +766,7 @@ __device__ __forceinline__ void finish_gram(const SkParams &p, int et, int nt) {
 // 93.3 vs 89.5 us per iteration with the sample).  The per-CTA sums are combined by the last CTA in
 // CTA order, so the value is deterministic.
 template <int FNP, bool QF = false>
-__global__ void __launch_bounds__(gemm_threads(FNP, QF), 1)
+__global__ void __launch_bounds__(gemm_threads(FNP, QF, kMaxGramThreads), 1)
     tc_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmQ, SkParams p) {
     const uintptr_t base = (reinterpret_cast<uintptr_t>(tc_dyn_smem) + 1023) & ~uintptr_t(1023);
@@ -792,7 +797,7 @@ __global__ void __launch_bounds__(gemm_threads(FNP, QF), 1)
     if (FNP == 0 && (int)blockIdx.x >= ctas) {  // no blocks of the product: a share of the Gram only
         griddep_wait();
         griddep_launch_dependents();
-        if (p.gram_out) finish_gram(p, threadIdx.x, gemm_threads(0));
+        if (p.gram_out) finish_gram(p, threadIdx.x, blockDim.x);
         return;
     }
     const long long T = (long long)p.tiles * p.kblocks;
@@ -1040,11 +1045,10 @@ __global__ void __launch_bounds__(gemm_threads(FNP, QF), 1)
         }
     } else if constexpr (FNP == 0) {
         // this CTA's share of the Gram matrix that the update kernel of the previous half-step left as
-        // partials (by the four draining warps it took longer than the product: 500 x 500, r = 100, 55.8 us
-        // an iteration against 44.8)
+        // partials
         griddep_wait();
         griddep_launch_dependents();
-        if (p.gram_out) finish_gram(p, threadIdx.x - kGemmThreads, 32 * kGramWarps);
+        if (p.gram_out) finish_gram(p, threadIdx.x - kGemmThreads, blockDim.x - kGemmThreads);
     } else {
       if (warp < 8) {
         griddep_wait();
@@ -1617,7 +1621,8 @@ __device__ __forceinline__ void upd_lds(const float *row, int g, float (&v)[TA])
 }
 
 // rows c0 .. c0 + ROWS - 1 of the factor, by NT threads; part: the index of their Gram partial (BF16 jobs:
-// of the first 16 rows'), sm: update_smem_bytes
+// of the first 16 rows'), sm: update_smem_bytes.  The slot lists do not change: they are read before the
+// wait for the kernel that fills the slots.
 template <int RP, int ROWS, int NT>
 __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part, float *sm) {
     constexpr int TA = RP / 16, RT = ROWS * 16 / NT;
@@ -1628,6 +1633,18 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
     const int tid = threadIdx.x;
     const int ncol = min(ROWS, p.cols - c0);
     const int r = p.r;
+    const int tile = c0 / 128, lrow0 = c0 % 128;
+    int s0 = p.slot0, s1 = p.slot0 + p.slots;
+    constexpr int kIds = 8;  // slots whose numbers are held (most tiles have fewer)
+    int ids[kIds];
+    if (p.slot_ptr && p.update) {
+        s0 = p.slot_ptr[tile];
+        s1 = p.slot_ptr[tile + 1];
+    }
+#pragma unroll
+    for (int q = 0; q < kIds; q++) ids[q] = p.slot_ptr && p.update ? p.slot_list[min(s0 + q, s1 - 1)] : min(s0 + q, s1 - 1);
+    griddep_wait();  // the GEMM's partial slots and Gram are complete
+    griddep_launch_dependents();
     // the old rows, zero outside r and ncol; a thread issues up to sixteen loads before it stores
     constexpr int XL = RP * ROWS / NT, XB = XL < 16 ? XL : 16;
 #pragma unroll 1
@@ -1663,31 +1680,37 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
             reinterpret_cast<float4 *>(Gs)[k] = __ldcg(reinterpret_cast<const float4 *>(p.G) + k);
         // numerators: the tile's slots summed in their order, four slots' loads of a thread together.
         // (Rows of a slot beyond the last are in bounds, the tile has 128; they are never stored.)
-        const int tile = c0 / 128, lrow0 = c0 % 128;
-        const int s0 = p.slot_ptr ? p.slot_ptr[tile] : p.slot0, s1 = p.slot_ptr ? p.slot_ptr[tile + 1] : p.slot0 + p.slots;
         constexpr int N4 = ROWS * RP / 4;
 #pragma unroll 1
         for (int k0 = 0; k0 < N4; k0 += 2 * NT) {
             const int ka = k0 + tid, kb = ka + NT;
-            const bool oa = ka < N4, ob = kb < N4;
+            const bool oa = ka < N4, ob = N4 > NT && kb < N4;
             float4 sa = make_float4(0.f, 0.f, 0.f, 0.f), sb = sa;
             auto add = [](float4 &s, const float4 &v) { s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; };
-#pragma unroll 1
-            for (int q0 = s0; q0 < s1; q0 += 4) {
-                float4 va[4], vb[4];
+            auto four = [&](const int (&id)[4], int live) {  // four slots, of which the first `live` count
+                float4 va[4], vb[4];  // (vb: only where a thread has two vectors)
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const int sq = min(q0 + q, s1 - 1), slot = p.slot_ptr ? p.slot_list[sq] : sq;
-                    const float4 *src = reinterpret_cast<const float4 *>(p.P + (size_t)slot * 128 * p.npad + lrow0 * RP);
+                    const float4 *src = reinterpret_cast<const float4 *>(p.P + (size_t)id[q] * 128 * p.npad + lrow0 * RP);
                     if (oa) va[q] = __ldcg(src + ka);
                     if (ob) vb[q] = __ldcg(src + kb);
                 }
 #pragma unroll
                 for (int q = 0; q < 4; q++)
-                    if (q0 + q < s1) {
+                    if (q < live) {
                         if (oa) add(sa, va[q]);
                         if (ob) add(sb, vb[q]);
                     }
+            };
+            const int ia[4] = {ids[0], ids[1], ids[2], ids[3]}, ib[4] = {ids[4], ids[5], ids[6], ids[7]};
+            four(ia, s1 - s0);
+            if (s1 - s0 > 4) four(ib, s1 - s0 - 4);
+#pragma unroll 1
+            for (int q0 = s0 + kIds; q0 < s1; q0 += 4) {
+                int id[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) id[q] = p.slot_ptr ? p.slot_list[min(q0 + q, s1 - 1)] : min(q0 + q, s1 - 1);
+                four(id, s1 - q0);
             }
             auto put = [&](int k, float4 v) {
                 const int c = k / (RP / 4), a = (k % (RP / 4)) * 4;
@@ -1713,7 +1736,7 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
         for (int i = 0; i < TA; i++)
 #pragma unroll
             for (int j = 0; j < RT; j++) den[i][j] = 0.f;
-#pragma unroll 4
+#pragma unroll(TA <= 3 ? 16 : 4)
         for (int b = 0; b < RP; b++) {
             float xb[RT], g[TA];
             lds_vec<RT>(Xs + b * LDX + gc * RT, xb);
@@ -1794,15 +1817,18 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
             for (int i = 0; i < TA; i++)
 #pragma unroll
                 for (int k = 0; k < TA; k++) acc[i][k] = 0.f;
-#pragma unroll 2
-            for (int c = c1; c < c1 + step; c++) {
-                float xa[TA], xb[TA];
-                upd_lds<TA>(Ns + c * LDN, ga, xa);
-                upd_lds<TA>(Ns + c * LDN, gb, xb);
+#pragma unroll 1
+            for (int cb = c1; cb < c1 + step; cb += 16) {
+#pragma unroll(TA <= 4 ? 16 : 2)
+                for (int c = cb; c < cb + 16; c++) {
+                    float xa[TA], xb[TA];
+                    upd_lds<TA>(Ns + c * LDN, ga, xa);
+                    upd_lds<TA>(Ns + c * LDN, gb, xb);
 #pragma unroll
-                for (int i = 0; i < TA; i++)
+                    for (int i = 0; i < TA; i++)
 #pragma unroll
-                    for (int k = 0; k < TA; k++) acc[i][k] = fmaf(xa[i], xb[k], acc[i][k]);
+                        for (int k = 0; k < TA; k++) acc[i][k] = fmaf(xa[i], xb[k], acc[i][k]);
+                }
             }
             if (H == 2 && p.Xs) {  // (G is read by no one any more: a barrier lies behind the denominators)
                 if (half == 1) {
@@ -1829,11 +1855,10 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
     }
 }
 
+// (rank 16: 48 registers, so that two fit beside a CTA of the product)
 template <int RP, int ROWS>
-__global__ void __launch_bounds__(upd_threads(RP)) tc_update_kernel(UpdParams p) {
+__global__ void __launch_bounds__(upd_threads(RP), RP <= 16 ? 5 : 1) tc_update_kernel(UpdParams p) {
     extern __shared__ __align__(16) float sm[];
-    griddep_wait();  // the GEMM's partial slots and Gram are complete
-    griddep_launch_dependents();
     update_rows<RP, ROWS, upd_threads(RP)>(p, blockIdx.x * ROWS, blockIdx.x * (p.Xs ? 1 : ROWS / kUpdGramRows), sm);
 }
 
@@ -2633,6 +2658,7 @@ struct TcGemm {
     int smem = 0;
     int smem_qf = 0;  // shared memory of the variant with the quality warps
     int fnp = 0;  // fused update rank (kernel template argument), 0 = separate update kernel
+    int gram = 0; // threads that finish the Gram (no fused update)
     int *slot_ptr = nullptr, *slot_list = nullptr;
     int *counters = nullptr;  // [tiles] arrivals, [tiles] readers done, [tiles] readers, [2] Gram assembly
     float *grams = nullptr;   // [grid][npad^2] per-CTA Gram partials of the factor this GEMM updates
@@ -2824,7 +2850,8 @@ static gpunmf_status setup_gemm(gpunmf_job *j, TcGemm &g, int rows, int K, int n
     // Where the product makes few CTAs, more of them share the Gram's npad^2 entries: 500 x 500, r = 100,
     // took 22.7 us a launch with the product's 16 CTAs alone (the Gram 15 of them).
     g.p.ctas = g.grid;
-    if (!fnp) g.grid = std::max(g.grid, std::min(j->tc->max_ctas, npad * npad / (gemm_threads(0) / 4)));
+    g.gram = fnp ? 0 : gram_threads(npad, g.p.ctas);
+    if (!fnp) g.grid = std::max(g.grid, std::min(j->tc->max_ctas, npad * npad / (gemm_threads(0, false, g.gram) / 4)));
     g.smem = 1024 + stages * stage_bytes + (2 * stages + 5) * 8 + 16 + (fnp ? 16 + fused_smem_bytes(fnp) : 0);
     // with the folded quality sample: two H-tile slots, eight more barriers, the warps' sums
     g.smem_qf = g.smem + 2 * 2 * npad * kBlockK * 2 + (4 + 2 * kQfSBufs) * 8 + 2 * kQfWarps * 8;
@@ -3619,7 +3646,7 @@ static cudaError_t launch_gemm_cfg(TcGemm &g, cudaLaunchConfig_t &cfg, bool qf) 
 static cudaError_t launch_gemm(TcGemm &g, cudaStream_t s, bool qf = false) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g.grid);
-    cfg.blockDim = dim3(gemm_threads(g.fnp, qf));
+    cfg.blockDim = dim3(gemm_threads(g.fnp, qf, g.gram));
     cfg.dynamicSmemBytes = qf ? g.smem_qf : g.smem;
     cfg.stream = s;
     cudaLaunchAttribute at[2];
