@@ -98,7 +98,7 @@ bool tc_quality_ready(const gpunmf_job *j);
 // whether the tensor-core quality kernel writes the job's pinned read-back word itself
 bool tc_quality_writes_host(const gpunmf_job *j);
 gpunmf_status tc_quality(gpunmf_job *j);
-// fused Euclidean jobs: the next H-step launch samples the quality itself (it also records the
+// fused Euclidean and KL jobs: the next H-step launch samples the quality itself (it also records the
 // job's quality event); false where it cannot
 bool tc_quality_fold(gpunmf_job *j);
 gpunmf_status tc_check(gpunmf_job *j);    // reads the kernels' error word (after a sync)

@@ -1910,6 +1910,10 @@ struct KlParams {
     int *tile_cnt, *tile_rd;          // per tile: partial products out, readers done (the last resets)
     const int *tile_readers;          // per tile: how many CTAs read it
     int *sum_cnt;                     // [2]: CTAs whose denominator entries are out; CTAs done (last resets)
+    // quality sample of the factors an H-step starts from, from the S it forms anyway (kernels with QF)
+    double *qpartial;                 // [grid]
+    int *qdone;                       // CTAs done (the last sums the partials in CTA order, resets it)
+    float *qout, *qout_host;          // the value: device word, and the pinned read-back word (or null)
     float *sum_part_out;              // [grid][npad] sums of this CTA's new rows (the next kernel's denominators)
 };
 
@@ -2089,8 +2093,9 @@ __device__ __forceinline__ void ring_next(int &i, uint32_t &ph, int n) {
 }
 
 
-// NK = npad / 16: the K16 steps of MMA1 (compile-time, so the MMA thread issues straight-line code)
-template <int NK>
+// NK = npad / 16: the K16 steps of MMA1 (compile-time, so the MMA thread issues straight-line code).
+// QF: the launch also samples the quality (a kernel of its own: the sums' registers spill in the other)
+template <int NK, bool QF = false>
 __global__ void __launch_bounds__(kKlThreads)
     tc_kl_gemm_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmA1,
                       const __grid_constant__ CUtensorMap tmF, KlParams p) {
@@ -2393,6 +2398,7 @@ __global__ void __launch_bounds__(kKlThreads)
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         int vi = 0, di = 0, seg = 0;
         uint32_t vph = 0, dph = 0;
+        double dlog = 0.0, ds = 0.0;  // the sample's sums: V log2(S + eps) and S
         for (long long b = lo; b < hi;) {
             const long long e = seg_end(b);
             bool ok = true;
@@ -2407,7 +2413,7 @@ __global__ void __launch_bounds__(kKlThreads)
                 tc_fence_after();
                 const uint32_t ta = tD1 + (uint32_t)(di * kKlBlockK + part * 32) + lane_off;
                 float sv[32];
-                {
+                if constexpr (!QF) {
                     float (&s0)[16] = *reinterpret_cast<float (*)[16]>(&sv[0]);
                     float (&s1)[16] = *reinterpret_cast<float (*)[16]>(&sv[16]);
                     tmem_ld16(ta, s0);
@@ -2421,7 +2427,12 @@ __global__ void __launch_bounds__(kKlThreads)
                 // the V stage is read (the arrive orders the loads before the producer's refill)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&vempty[vi]);
-                tmem_ld_wait();
+                if constexpr (QF) {
+                    tmem_ld16_sync(ta, *reinterpret_cast<float (*)[16]>(&sv[0]));
+                    tmem_ld16_sync(ta + 16, *reinterpret_cast<float (*)[16]>(&sv[16]));
+                } else {
+                    tmem_ld_wait();
+                }
                 uint32_t rr[16];
 #pragma unroll
                 for (int cc = 0; cc < 4; cc++) {
@@ -2443,6 +2454,27 @@ __global__ void __launch_bounds__(kKlThreads)
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&rfull[di]);
+                if constexpr (QF) {
+                    // the sample, behind the chain: the second product has its R already.  (As a launch of
+                    // its own it streamed V and formed W H again: 45 us an iteration of 140 at 16384 x
+                    // 4096, r = 128.)  Zero-padded entries add 0.
+                    float plog[4] = {0.f, 0.f, 0.f, 0.f}, ps[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int cc = 0; cc < 4; cc++) {
+                        const __nv_bfloat162 *v2 = reinterpret_cast<const __nv_bfloat162 *>(&vraw[cc]);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const float2 vf = __bfloat1622float2(v2[q]);
+                            const int j = cc * 8 + 2 * q;
+                            plog[q] = fmaf(vf.x, lg2_approx(sv[j] + eps_pos), plog[q]);
+                            plog[q] = fmaf(vf.y, lg2_approx(sv[j + 1] + eps_pos), plog[q]);
+                            ps[q] += sv[j];
+                            ps[q] += sv[j + 1];
+                        }
+                    }
+                    dlog += (double)((plog[0] + plog[1]) + (plog[2] + plog[3]));
+                    ds += (double)((ps[0] + ps[1]) + (ps[2] + ps[3]));
+                }
                 ring_next(vi, vph, p.sv);
                 ring_next(di, dph, p.nb);
             }
@@ -2471,6 +2503,43 @@ __global__ void __launch_bounds__(kKlThreads)
             }
             seg++;
             b = e;
+        }
+        if constexpr (QF) {  // (the sixteen warps leave the loop together)
+            double *qred = reinterpret_cast<double *>(red + 32);  // [2][16]
+            const int qw = warp - 2;
+            dlog = warp_sum(dlog);
+            ds = warp_sum(ds);
+            if (lane == 0) {
+                qred[qw] = dlog;
+                qred[kKlEpiWarps + qw] = ds;
+            }
+            asm volatile("bar.sync 3, 512;" ::: "memory");
+            if (qw == 0) {
+                double l = 0.0, sm = 0.0;
+                for (int w = 0; w < kKlEpiWarps; w++) {
+                    l += qred[w];
+                    sm += qred[kKlEpiWarps + w];
+                }
+                int last = 0;
+                if (lane == 0) {
+                    p.qpartial[blockIdx.x] = 0.30102999566398120 * l - sm;  // log10(x) = log2(x) log10(2)
+                    last = atom_acq_rel_add(p.qdone, 1) == (int)gridDim.x - 1;
+                }
+                if (__shfl_sync(0xffffffffu, last, 0)) {
+                    // the last CTA: the partials in CTA order (lane-strided, then a fixed tree)
+                    double q = 0.0;
+                    for (int c = lane; c < (int)gridDim.x; c += 32) q += __ldcg(p.qpartial + c);
+                    q = warp_sum(q);
+                    if (lane == 0) {
+                        p.qout[0] = (float)q;
+                        if (p.qout_host) {
+                            p.qout_host[0] = (float)q;
+                            __threadfence_system();
+                        }
+                        *p.qdone = 0;
+                    }
+                }
+            }
         }
     }
     __syncthreads();
@@ -2695,7 +2764,7 @@ struct TcState {
     int qgrid = 0, qsmem = 0;
     float *GP_w = nullptr, *GP_h = nullptr;   // per-CTA Gram partials of the update kernels
     int gp_w_count = 0, gp_h_count = 0;
-    bool qfold = false;        // the quality sample can ride on the H-step (fused Euclidean jobs)
+    bool qfold = false;        // the quality sample can ride on the H-step (fused Euclidean and KL jobs)
     bool qfold_armed = false;  // the next H-step carries it
     int max_ctas = 0;                         // CTAs per launch: the SMs, or fewer (gpunmf_set_grid_limit)
 };
@@ -3053,7 +3122,9 @@ static cudaError_t set_kl_smem_once() {
         result = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
 #define KLATTR(NK)                                                                                     \
     if (result == cudaSuccess)                                                                         \
-        result = cudaFuncSetAttribute(tc_kl_gemm_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        result = cudaFuncSetAttribute(tc_kl_gemm_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin); \
+    if (result == cudaSuccess)                                                                         \
+        result = cudaFuncSetAttribute(tc_kl_gemm_kernel<NK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         KLATTR(1) KLATTR(2) KLATTR(3) KLATTR(4) KLATTR(5) KLATTR(6) KLATTR(7) KLATTR(8)
 #undef KLATTR
     });
@@ -3230,7 +3301,7 @@ __global__ void kl_row_sums_kernel(const float *__restrict__ X, int is_w, long l
     }
 }
 
-static cudaError_t launch_kl_gemm(KlGemm &g, cudaStream_t s) {
+static cudaError_t launch_kl_gemm(KlGemm &g, cudaStream_t s, bool qf = false) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g.grid);
     cfg.blockDim = dim3(kKlThreads);
@@ -3244,7 +3315,9 @@ static cudaError_t launch_kl_gemm(KlGemm &g, cudaStream_t s) {
     auto launch = [&]() -> cudaError_t {
         switch (g.p.npad / 16) {
 #define KLCASE(NK) \
-    case NK: return cudaLaunchKernelEx(&cfg, tc_kl_gemm_kernel<NK>, g.tmV, g.tmA1, g.tmF, g.p);
+    case NK:          \
+        return qf ? cudaLaunchKernelEx(&cfg, tc_kl_gemm_kernel<NK, true>, g.tmV, g.tmA1, g.tmF, g.p) \
+                  : cudaLaunchKernelEx(&cfg, tc_kl_gemm_kernel<NK>, g.tmV, g.tmA1, g.tmF, g.p);
             KLCASE(1) KLCASE(2) KLCASE(3) KLCASE(4) KLCASE(5) KLCASE(6) KLCASE(7) KLCASE(8)
 #undef KLCASE
         }
@@ -3414,6 +3487,11 @@ static gpunmf_status setup_quality(gpunmf_job *j) {
         return GPUNMF_ERR_CUDA;
     }
     q.partial = j->red;
+    // KL jobs sample it in their H-step, which forms the same W H
+    if (rule_is_kl(j->rule)) {
+        t->qfold = (size_t)t->kh.grid <= j->red_cap;
+        return GPUNMF_OK;
+    }
     // fused Euclidean jobs with an H-step sample the quality inside it (the H-step streams the same V)
     TcGemm &g = t->gh;
     if (g.fnp && j->rule != GPUNMF_ADDITIVE_EUCLIDEAN_FIXED_H && g.p.bps == 2 && (size_t)g.grid <= j->red_cap &&
@@ -3670,9 +3748,21 @@ gpunmf_status tc_iterate(gpunmf_job *j, bool updateW) {
         // (additive KL: the same numerator, applied as H + (H / max(colsum W, eps)) (num - colsum W))
         // (one launch per half-step where the update is fused into the product kernel's tail)
         const bool fused = t->kh.p.X != nullptr;
+        const bool qf = t->qfold_armed;  // this H-step also samples the quality
+        t->qfold_armed = false;
+        t->kh.p.qpartial = j->red;
+        t->kh.p.qdone = t->qp.done;
+        t->kh.p.qout = t->qp.out;
+        t->kh.p.qout_host = t->qp.out_host;
         mark_begin(j);
-        GPUNMF_CUDA_TRY(launch_kl_gemm(t->kh, s));
+        GPUNMF_CUDA_TRY(launch_kl_gemm(t->kh, s, qf));
         mark_end(j);
+        if (qf) {
+            if (!tc_quality_writes_host(j))
+                GPUNMF_CUDA_TRY(cudaMemcpyAsync(j->h_quality(), j->d_quality, sizeof(float), cudaMemcpyDeviceToHost, s));
+            GPUNMF_CUDA_TRY(cudaEventRecord(j->qev, s));
+            j->q_pending = true;
+        }
         if (!fused) GPUNMF_CUDA_TRY(launch_kl_update(kl_params_h(j, 1), t->npad, false, s));
         j->launches += fused ? 1 : 2;
         if (!updateW) return GPUNMF_OK;
