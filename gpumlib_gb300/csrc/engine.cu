@@ -335,6 +335,14 @@ static gpunmf_status job_upload(gpunmf_job *j, const float *V, const float *W, c
 // rule: an iteration samples only if the previous read-back is complete
 // (nmf_base.h:71, cudaStreamQuery on the read-back's stream), and never waits.
 // ------------------------------------------------------------------------
+gpunmf_status job_quality_sampled(gpunmf_job *j, bool wrote_host) {
+    if (!wrote_host)
+        GPUNMF_CUDA_TRY(cudaMemcpyAsync(j->h_quality(), j->d_quality, sizeof(float), cudaMemcpyDeviceToHost, j->stream));
+    GPUNMF_CUDA_TRY(cudaEventRecord(j->qev, j->stream));
+    j->q_pending = true;
+    return GPUNMF_OK;
+}
+
 static gpunmf_status quality_step(gpunmf_job *j, bool fused_wh) {
     if (j->q_interval == 0) return GPUNMF_OK;
     if (j->q_interval > 0 && (j->iter_count % j->q_interval) != 0) return GPUNMF_OK;
@@ -373,12 +381,9 @@ static gpunmf_status quality_step(gpunmf_job *j, bool fused_wh) {
         return GPUNMF_OK;
     }
     if (j->precision == GPUNMF_FP32 && j->sp) {  // one launch, which writes the read-back word too
+        if (sp_quality_fold(j)) return GPUNMF_OK;
         TRY_STATUS(sp_quality(j));
-        if (!sp_quality_writes_host(j))
-            GPUNMF_CUDA_TRY(cudaMemcpyAsync(j->h_quality(), j->d_quality, sizeof(float), cudaMemcpyDeviceToHost, s));
-        GPUNMF_CUDA_TRY(cudaEventRecord(j->qev, s));
-        j->q_pending = true;
-        return GPUNMF_OK;
+        return job_quality_sampled(j, sp_quality_writes_host(j));
     }
     if (fused_wh) {
         GPUNMF_CUDA_TRY(wh_quality_f32(n, m, r, j->W, j->H, j->V, j->eps, j->red, s));

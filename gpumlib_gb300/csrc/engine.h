@@ -116,6 +116,9 @@ gpunmf_status sp_prepare(gpunmf_job *j, bool residual_only);  // after V, W, H a
 gpunmf_status sp_iterate(gpunmf_job *j, bool updateW);
 gpunmf_status sp_quality(gpunmf_job *j);
 bool sp_quality_writes_host(const gpunmf_job *j);
+bool sp_quality_fold(gpunmf_job *j);
+// after a launch that sampled the quality: its read-back (unless the launch wrote the host's word) and event
+gpunmf_status job_quality_sampled(gpunmf_job *j, bool wrote_host);
 gpunmf_status sp_residual(gpunmf_job *j, double *d_out);
 void sp_destroy(gpunmf_job *j);
 void job_residual_ready(gpunmf_job *j);  // before the first job_residual (may allocate)

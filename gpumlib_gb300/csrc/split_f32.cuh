@@ -13,13 +13,14 @@
 //                way from shared memory to TMEM; B = the other factor's chunk (three BF16 copies)
 //   kSpKl        slots of  W'(V ./ (WH + eps)): a first product forms S = the chunk of W H in TMEM,
 //                and A = V / (S + eps) (- 1 for the additive rule), cut the same way; W H is not stored
+//   kSpKlQuality the same H-step, which also sums the quality of the factors it starts from
 //   kSpQuality   sum V log10(WH + eps) - WH;  kSpResidual  sum (V - WH)^2 and sum V^2
 // V is read as it is (FP32, column-major, both half-steps from the one copy): along K it is
 // contiguous for the H-step (rows u) and strided for the W-step (rows i); both arrive by TMA.
 // What bounds it: V's 4 bytes an element from HBM (39.5 us at 8192 x 8192) against
 // 24 MMAs of 128 x npad x 16 a chunk (21.6 us there at r = 64, 43 us at r = 128).
 
-enum SpMode { kSpEuclid = 0, kSpKl = 1, kSpQuality = 2, kSpResidual = 3 };
+enum SpMode { kSpEuclid = 0, kSpKl = 1, kSpKlQuality = 2, kSpQuality = 3, kSpResidual = 4 };
 
 constexpr int kSpChunk = 64;                       // K per chunk
 constexpr int kSpVBytes = kTileM * kSpChunk * 4;   // 32 KB of V a chunk
@@ -200,9 +201,10 @@ template <int NPC, int MODE>
 __global__ void __launch_bounds__(kSpThreads, 1)
     sp_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmF, SpParams p) {
     constexpr bool kFirst = MODE != kSpEuclid;   // has the first product S
+    constexpr bool kKl = MODE == kSpKl || MODE == kSpKlQuality, kSum = MODE >= kSpKlQuality;  // ends in a sum
     constexpr bool kReduce = MODE >= kSpQuality;  // ends in a reduction, has no second product
     constexpr int ND1 = kReduce ? 2 : 1;          // S buffers (64 columns)
-    constexpr int NR = MODE == kSpKl && NPC == 128 ? 1 : 2;  // A buffers (3 x 32 columns)
+    constexpr int NR = kKl && NPC == 128 ? 1 : 2;  // A buffers (3 x 32 columns)
     constexpr int ND2 = NR;                       // accumulators (NPC columns)
     const uintptr_t base = (reinterpret_cast<uintptr_t>(tc_dyn_smem) + 1023) & ~uintptr_t(1023);
     const int fBytes = p.nbox * kSpFBox;
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
     if (!kReduce && (int)blockIdx.x >= p.ctas) {
         griddep_wait();
         griddep_launch_dependents();
-        sp_finish_other<MODE>(p, threadIdx.x, kSpThreads);
+        sp_finish_other<kKl ? kSpKl : MODE>(p, threadIdx.x, kSpThreads);
         return;
     }
     const long long lo = (long long)blockIdx.x * T / p.ctas;
@@ -447,6 +449,29 @@ __global__ void __launch_bounds__(kSpThreads, 1)
 #pragma unroll
             for (int c = 0; c < NC; c++) acc[c] = 0.f;
         }
+        // the quality's terms of sixteen columns
+        auto sample = [&](const float (&v)[16], const float (&s)[16], int klim) {
+            if constexpr (MODE == kSpQuality || MODE == kSpKlQuality) {
+                uint32_t range = 0;
+                float2 l[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++)
+                    l[c] = log10_pair(add2(make_float2(s[2 * c], s[2 * c + 1]), both(p.eps)), range);
+                if (!__any_sync(0xffffffffu, klim < 16 || range >= 0x7F000000u)) {
+#pragma unroll
+                    for (int c = 0; c < 8; c++) {
+                        const float2 s2 = make_float2(s[2 * c], s[2 * c + 1]);
+                        two_sum(qs, qc, sub2(mul2(make_float2(v[2 * c], v[2 * c + 1]), l[c]), s2));
+                    }
+                } else {  // the edge of V, or a sum that is zero, subnormal, infinite or NaN
+#pragma unroll
+                    for (int c = 0; c < 16; c++)
+                        if (c < klim)
+                            two_sum(qs, qc, make_float2(v[c] * log10f(s[c] + p.eps) - s[c], 0.f));
+                }
+                __syncwarp();
+            }
+        };
         // adds the oldest undrained chunk's product; the last chunk of a segment completes a slot
         auto drain = [&](bool last) -> bool {
             if constexpr (!kReduce) {
@@ -539,7 +564,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
                 // (V is finite, or the update kernel forms the sums again)
 #pragma unroll
                 for (int c = 0; c < 8; c++) cut_pair(v[2 * c], v[2 * c + 1], w0[c], w1[c], w2[c]);
-            } else if constexpr (MODE == kSpKl) {
+            } else if constexpr (kKl) {
                 // V / (S + eps): the quotient by the approximate reciprocal and one residual step
                 // (Markstein), which a division in range rounds like the operator but for rare last
                 // bits, without its branch; a warp with any other division takes the operator
@@ -575,24 +600,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
                     __syncwarp();
                 }
             } else if constexpr (MODE == kSpQuality) {
-                uint32_t range = 0;
-                float2 l[8];
-#pragma unroll
-                for (int c = 0; c < 8; c++)
-                    l[c] = log10_pair(add2(make_float2(s[2 * c], s[2 * c + 1]), both(p.eps)), range);
-                if (!__any_sync(0xffffffffu, klim < 16 || range >= 0x7F000000u)) {
-#pragma unroll
-                    for (int c = 0; c < 8; c++) {
-                        const float2 s2 = make_float2(s[2 * c], s[2 * c + 1]);
-                        two_sum(qs, qc, sub2(mul2(make_float2(v[2 * c], v[2 * c + 1]), l[c]), s2));
-                    }
-                } else {  // the edge of V, or a sum that is zero, subnormal, infinite or NaN
-#pragma unroll
-                    for (int c = 0; c < 16; c++)
-                        if (c < klim)
-                            two_sum(qs, qc, make_float2(v[c] * log10f(s[c] + p.eps) - s[c], 0.f));
-                }
-                __syncwarp();
+                sample(v, s, klim);
             } else {
                 // (v - s)^2 and v^2 with what FP32 drops of them (zeros beyond the last row and K)
                 if (klim < 16) {
@@ -637,6 +645,8 @@ __global__ void __launch_bounds__(kSpThreads, 1)
                 if constexpr (!kReduce) mbar_arrive(&rfull[rb]);
                 mbar_arrive(&vempty[vs]);
             }
+            // (the sample comes behind the chain: the second product has its operand)
+            if constexpr (MODE == kSpKlQuality) sample(v, s, t * kTileM + row < p.a1_rows ? klim : 0);
             ring_next(vs, vph, p.sv);
             ring_next(rb, rph, NR);
             if (++kk == p.kchunks) {
@@ -652,7 +662,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
             if (j > 0 && !drain(false)) break;
             if (j + 1 == nblk) drain(true);
         }
-        if constexpr (kReduce) {
+        if constexpr (kSum) {
             double a = ((double)qs.x + (double)qc.x) + ((double)qs.y + (double)qc.y);
             double b = ((double)ws.x + (double)wc.x) + ((double)ws.y + (double)wc.y);
             a = warp_sum(a);
@@ -666,10 +676,10 @@ __global__ void __launch_bounds__(kSpThreads, 1)
         // two more warps finish what the update kernel needs of the other factor
         griddep_wait();
         griddep_launch_dependents();
-        sp_finish_other<MODE>(p, threadIdx.x - (kSpThreads - 64), 64);
+        sp_finish_other<kKl ? kSpKl : MODE>(p, threadIdx.x - (kSpThreads - 64), 64);
     }
     __syncthreads();
-    if constexpr (kReduce) {
+    if constexpr (kSum) {
         if (threadIdx.x == 0) {
             double a = 0.0, b = 0.0;
             for (int w = 0; w < 16; w++) {
@@ -679,14 +689,14 @@ __global__ void __launch_bounds__(kSpThreads, 1)
             constexpr int kTerms = MODE == kSpResidual ? 2 : 1;
             p.reduce[kTerms * blockIdx.x] = a;
             if constexpr (kTerms == 2) p.reduce[kTerms * blockIdx.x + 1] = b;
-            reinterpret_cast<volatile int *>(red)[0] = atom_acq_rel_add(p.done, 1) == (int)gridDim.x - 1;
+            reinterpret_cast<volatile int *>(red)[0] = atom_acq_rel_add(p.done, 1) == p.ctas - 1;
         }
         __syncthreads();
         if (warp == 0 && reinterpret_cast<volatile int *>(red)[0]) {
             // the last CTA: the partials in CTA order (lane-strided, then a fixed tree)
             constexpr int kTerms = MODE == kSpResidual ? 2 : 1;
             double a = 0.0, b = 0.0;
-            for (int c = lane; c < (int)gridDim.x; c += 32) {
+            for (int c = lane; c < p.ctas; c += 32) {
                 a += __ldcg(p.reduce + kTerms * c);
                 if constexpr (kTerms == 2) b += __ldcg(p.reduce + kTerms * c + 1);
             }
@@ -754,6 +764,7 @@ struct SpState {
     float *S_w = nullptr, *S_h = nullptr, *SP_w = nullptr, *SP_h = nullptr;  // KL: sums and their partials
     double *reduce = nullptr;
     int *err = nullptr, *done = nullptr;
+    bool sample = false;        // the next KL H-step sums the quality
     char *arena = nullptr;      // all of the above: one allocation
     gpunmf::SpGemm gh, gw, gq;  // H-step, W-step, quality / residual
 };
@@ -900,6 +911,8 @@ static cudaError_t sp_set_smem(int optin) {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(sp_kernel<NPC, kSpKl>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(sp_kernel<NPC, kSpKlQuality>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(sp_kernel<NPC, kSpQuality>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(sp_kernel<NPC, kSpResidual>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
@@ -1035,6 +1048,8 @@ gpunmf_status sp_create(gpunmf_job *j, bool residual_only) {
     st = sp_map_v(&t->gw.tmV, V, n, m, ldv, false);
     if (st == GPUNMF_OK) st = sp_map_f(&t->gw.tmF, t->Hs, m, np);
     t->gw.p.A1 = t->Ws; t->gw.p.a1_part = (long long)n * np; t->gw.p.a1_rows = n;
+    t->gh.p.reduce = t->reduce; t->gh.p.done = t->done;
+    t->gh.p.qout = t->gq.p.qout; t->gh.p.qout_host = t->gq.p.qout_host;
     if (kl) {
         t->gh.p.sum_partials = t->SP_w; t->gh.p.sum_out = t->S_w; t->gh.p.sum_count = ceil_div(n, kKlUpdColsW);
         t->gw.p.sum_partials = t->SP_h; t->gw.p.sum_out = t->S_h; t->gw.p.sum_count = ceil_div(m, kKlUpdColsH);
@@ -1094,6 +1109,14 @@ gpunmf_status sp_prepare(gpunmf_job *j, bool residual_only) {
     return GPUNMF_OK;
 }
 
+bool sp_quality_writes_host(const gpunmf_job *j) { return j->sp->gq.p.qout_host != nullptr; }
+
+// KL jobs: the next H-step takes the sample (it records the job's quality event)
+bool sp_quality_fold(gpunmf_job *j) {
+    j->sp->sample = rule_is_kl(j->rule);
+    return j->sp->sample;
+}
+
 gpunmf_status sp_iterate(gpunmf_job *j, bool updateW) {
     SpState *t = j->sp;
     const bool kl = rule_is_kl(j->rule);
@@ -1103,15 +1126,21 @@ gpunmf_status sp_iterate(gpunmf_job *j, bool updateW) {
         if (w ? !updateW : j->rule == GPUNMF_ADDITIVE_EUCLIDEAN_FIXED_H) continue;
         const SpGemm &g = w ? t->gw : t->gh;
         mark_begin(j);
-        GPUNMF_CUDA_TRY(kl ? sp_launch<kSpKl>(t, g, j->stream) : sp_launch<kSpEuclid>(t, g, j->stream));
+        const bool sample = w == 0 && t->sample;  // a KL H-step
+        GPUNMF_CUDA_TRY(!kl      ? sp_launch<kSpEuclid>(t, g, j->stream)
+                        : sample ? sp_launch<kSpKlQuality>(t, g, j->stream)
+                                 : sp_launch<kSpKl>(t, g, j->stream));
         mark_end(j);
+        if (sample) {
+            t->sample = false;
+            gpunmf_status q = job_quality_sampled(j, sp_quality_writes_host(j));
+            if (q != GPUNMF_OK) return q;
+        }
         GPUNMF_CUDA_TRY(sp_update(j, w != 0, 1));
         j->launches += 2;
     }
     return GPUNMF_OK;
 }
-
-bool sp_quality_writes_host(const gpunmf_job *j) { return j->sp->gq.p.qout_host != nullptr; }
 
 // The quality of the current factors into j->d_quality, and the pinned read-back word.
 gpunmf_status sp_quality(gpunmf_job *j) {
