@@ -868,7 +868,8 @@ size_t sp_footprint(int rule, int n, int m, int r, bool residual_only) {
 }
 
 // V (n x m FP32, column stride ld): boxes of 32 rows i x 128 columns u, 128-byte swizzled (K along i),
-// or of 128 rows x 64 columns (K along u)
+// or of 128 rows x 64 columns (K along u).  L2 sectors promoted to 128 bytes: 256 made batches, whose
+// columns start anywhere, read 583 MB for 448 of V (342 us an iteration of 768 uneven ones, 331 so)
 static gpunmf_status sp_map_v(CUtensorMap *mp, const float *V, uint64_t n, uint64_t m, uint64_t ld, bool k_contig) {
     auto fn = encode_fn();
     cuuint64_t dims[2] = {n, m};
@@ -878,7 +879,7 @@ static gpunmf_status sp_map_v(CUtensorMap *mp, const float *V, uint64_t n, uint6
     CUresult r = fn ? fn(mp, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(V), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE,
                          k_contig ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
                     : CUDA_ERROR_NOT_SUPPORTED;
     if (r != CUDA_SUCCESS) {
         set_error("cuTensorMapEncodeTiled (FP32 V) failed (%d)", (int)r);
