@@ -57,10 +57,10 @@ GENERATOR = (" (project generator, gpumlib_gb300/inputs.py: splitmix64 counters 
              "gamma, Box-Muller normal, inversion / PTRS Poisson)")
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from the committed ncu
-# captures of this workload (one --set full capture per precision, see the profiles
+# captures of this workload (one capture per precision, see the profiles
 # directory): tc_gemm_sk_kernel<64> with the update fused, mean of an H-step and a W-step launch,
-# 138.76 MB + 3.75 MB; gemm_f32_kernel (W'V, 19 split-K slices) 275.49 MB + 25.29 MB.
-NCU_TRAFFIC_PER_LAUNCH = {"bf16": 142.51e6, "fp32": 300.78e6}
+# 138.76 MB + 3.75 MB; sp_kernel<64, 0> (W'V and V H' from FP32 V) 280.03 MB + 3.17 MB.
+NCU_TRAFFIC_PER_LAUNCH = {"bf16": 142.51e6, "fp32": 283.20e6}
 # The same for the KL workload's fused product (tc_kl_gemm_kernel<8>, mean of an H-step and a
 # W-step launch: 139.87 MB + 3.94 MB).
 KL_NCU_TRAFFIC_PER_LAUNCH = {"bf16": 143.81e6}
@@ -351,8 +351,8 @@ def run_ours(args, rank, world, local, dist):
         # factor read (FP32), written (FP32) and written again as BF16
         per_launch_bytes = n * m * 2 + n * r * 2 + m * r * (4 + 4 + 2)
     else:
-        # the W'V product: V, W and the FP32 partial products of H's shape
-        per_launch_bytes = n * m * 4 + (n * r + r * m) * 4 + r * m * 4
+        # the product from FP32 V: V, the other factor's three BF16 parts, the FP32 partial products
+        per_launch_bytes = n * m * 4 + n * r * 6 + r * m * 4
     kl = max(1, t["kernel_launches"])
     isolated_ms = t["kernel_ms"] / kl
     if t["launches"] == tk["kernel_launches"]:
@@ -370,9 +370,14 @@ def run_ours(args, rank, world, local, dist):
         roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                     "frac": round(achieved / hbm, 4), "peak_source": src,
                     "kernel": "half-step kernel: V-streaming product with the update fused (tc_gemm_sk_kernel)"}
+    elif r <= 128:
+        # products of BF16 parts on the tensor cores at FP32 accuracy: V's bytes bound them
+        roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
+                    "frac": round(achieved / hbm, 4), "peak_source": src,
+                    "kernel": "V-streaming product W'V / V H' of three-part operands (sp_kernel)"}
     else:
-        # the FP32 product is bound by the CUDA cores' FMA rate (8.6 GFLOP against 268 MB of V: 32
-        # flop per byte), so its roofline is the FP32 peak, computed (no measured figure exists)
+        # the FP32 product is bound by the CUDA cores' FMA rate, so its roofline is the FP32 peak, computed
+        # (no measured figure exists)
         mhz = peak_sm_mhz()
         fp32_peak = FP32_SMS * 128 * 2 * mhz * 1e6 / 1e12
         tfs = 2.0 * n * m * r / (avg_ms / 1e3) / 1e12
@@ -614,7 +619,7 @@ def run_batched(args, rank, world, local, dist):
         d2h = sum(w.nbytes + h.nbytes for w, h in outs)
         e2e = {"value": round(world * count / e2e_s, 1), "unit": "jobs/s", "h2d_bytes_per_step": h2d,
                "d2h_bytes_per_step": d2h,
-               "note": "a step is the whole batch: create from host (H2D), one persistent launch, all W/H read back"}
+               "note": "a step is the whole batch: create from host (H2D), all iterations, all W/H read back"}
     b.close()
     # comparison: one job per instance through the plain FP32 job API (a sample, largest and smallest mixed)
     sample = [insts[k] for k in range(0, count, max(1, count // args.baseline_sample))][:args.baseline_sample]
@@ -633,13 +638,15 @@ def run_batched(args, rank, world, local, dist):
                       "iters": iters, "rule": "euclidean", "precision": "fp32",
                       "l2": "each step re-reads every instance's V 2x per iteration; working set %.2f GB > L2" %
                             (sum(d["V"].nbytes for d in insts) / 1e9)},
-           "clocks": clk.summary(), "gpu_launches": args.steps,
+           # product and update of each half-step, shared by all instances
+           "clocks": clk.summary(), "gpu_launches": 4 * iters * args.steps,
            "roofline": {"bound": "fp32-simt", "achieved": round(2 * total_madds / (ms / 1e3) / 1e12, 2),
                         "peak": round(fp32_peak, 1), "unit": "TFLOP/s",
                         "frac": round(2 * total_madds / (ms / 1e3) / 1e12 / fp32_peak, 4),
                         "peak_source": "computed: %d SMs x 128 FP32 lanes x 2 flop x %.0f MHz (no measured FP32 "
                                        "figure exists for this GPU)" % (FP32_SMS, fp32_mhz),
-                        "note": "FP32 CUDA-core arithmetic; V served mostly from L2 (instances in flight)"},
+                        "note": "the FP32 CUDA cores' peak for comparison: the products run on the tensor cores, and V "
+                                "(two reads an iteration) bounds them"},
            "autotune": {"%d/%d" % k: v[0] for k, v in table.items()}, "autotune_s": round(tune_s, 2),
            "create_s": round(create_s, 2),
            "residual": {"median": float(np.median(res)), "max": float(np.max(res))},

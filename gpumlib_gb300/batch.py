@@ -1,8 +1,9 @@
 """Batched small factorisations and their tile autotuner (over the C ABI).
 
-``Batch`` holds thousands of uneven Euclidean instances on the device and
-runs all of them in one persistent, graph-captured launch
-(gpumlib_gb300/csrc/batch.cu).  ``autotune`` times every tile configuration
+``Batch`` holds thousands of uneven Euclidean instances on the device and runs all of them at once: every
+half-step's launches shared by all instances (gpumlib_gb300/csrc/split_batch.cuh), or, where that is
+faster, one persistent, graph-captured launch with one CTA per instance
+(gpumlib_gb300/csrc/batch.cu).  ``autotune`` (of use for the latter) times every tile configuration
 of the matching rank class on a sample of each (rank class, size) bucket and
 assigns the fastest to every instance of that bucket.
 """

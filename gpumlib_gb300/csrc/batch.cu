@@ -1,6 +1,7 @@
 // Batched multiplicative-update NMF: thousands of small, uneven Euclidean
 // factorisations in one persistent launch, and FacesNMF's grouped training on
-// top of it (end of file).
+// top of it (end of file).  Batches for which launches shared by all instances are faster run those
+// instead (split_batch.cuh, spb_better).
 //
 // The reference's nearest equivalent is FacesNMF's grouped training
 // (src/examples/FacesNMF/FacesNMFDlg.cpp:582-656), which builds one NMF
@@ -14,8 +15,7 @@
 //                                     H update, and the chunk's part of H H'
 //   W-step, per chunk of BC rows:     V H' chunk (streaming V), den = W G_H,
 //                                     W update, and the chunk's part of W'W
-// so each iteration reads V exactly twice (from L2: a few hundred instances
-// in flight fit in the 129 MB L2) and W, H a few times.  Arithmetic is FP32
+// so each iteration reads V exactly twice and W, H a few times.  Arithmetic is FP32
 // on the CUDA cores, the same rule and order as the plain drop-in path
 // (nmf_multiplicative_euclidian.cpp:29-67, nmf_kernels.cu:43-47).
 //
@@ -673,8 +673,8 @@ gpunmf_status gpunmf_batch_destroy(gpunmf_batch *b) {
     return GPUNMF_OK;
 }
 
-// Run `iters` iterations of every instance: one persistent launch, captured in a CUDA graph
-// (re-captured when iters changes) and replayed.  Returns without waiting.
+// Run `iters` iterations of every instance: the shared half-step launches, or one persistent launch,
+// captured in a CUDA graph (re-captured when iters changes) and replayed.  Returns without waiting.
 gpunmf_status gpunmf_batch_run(gpunmf_batch *b, int iters) {
     if (!b || iters < 0) return GPUNMF_ERR_INVALID;
     if (iters == 0) return GPUNMF_OK;

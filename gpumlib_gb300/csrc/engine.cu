@@ -15,8 +15,8 @@
 //   additive KL (src/algorithms/nmf/nmf_additive_divergence.cpp:29-51)
 //     WH = W H; quality(WH); H <- max(0, H + (H ./ max(colsum W, eps)) .* W' (V./(WH+eps) - 1));
 //     [WH = W H; W <- max(0, W + (W ./ max(rowsum H, eps)) .* (V./(WH+eps) - 1) H')]
-// with the product arithmetic chosen per job: FP32 CUDA cores (the drop-in
-// path) or BF16 tensor cores (tc_kernels.cu).
+// with the product arithmetic chosen per job: FP32 accuracy (the drop-in path; up to rank 128 on the
+// tensor cores, split_f32.cuh, above on the CUDA cores) or BF16 tensor cores (tc_kernels.cu).
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -420,7 +420,7 @@ void mark_end(gpunmf_job *j) {
 }
 
 // ------------------------------------------------------------------------
-// FP32 iterations
+// FP32 iterations on the CUDA cores (ranks above 128)
 // ------------------------------------------------------------------------
 static gpunmf_status iterate_euclid_f32(gpunmf_job *j, bool updateW) {
     const int n = j->n, m = j->m, r = j->r;

@@ -1,4 +1,5 @@
-// FP32 CUDA-core kernels of the plain (drop-in) NMF path.
+// FP32 CUDA-core kernels: the plain NMF path above rank 128 (split_f32.cuh has the others), the
+// kernel-level entry points, W H itself and small residuals.
 //
 // The reference runs its factor products through cuBLAS SGEMM
 // (src/memory/DeviceMatrix.h:195-227) and its updates through the kernels of

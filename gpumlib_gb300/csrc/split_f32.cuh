@@ -8,8 +8,8 @@
 // as with the FP32 FMA products this replaces (the tests hold them to the same bounds), at
 // 6 / 1900 of a flop's time instead of 1 / 80.
 //
-// One kernel, four modes, all over 128-row tiles and 64-wide chunks of K:
-//   kSpEuclid    slots of  V' W (H-step) or V H' (W-step):  A = the V chunk, cut by eight warps on its
+// One kernel, five modes, all over 128-row tiles and 64-wide chunks of K:
+//   kSpEuclid    slots of  V' W (H-step) or V H' (W-step):  A = the V chunk, cut by sixteen warps on its
 //                way from shared memory to TMEM; B = the other factor's chunk (three BF16 copies)
 //   kSpKl        slots of  W'(V ./ (WH + eps)): a first product forms S = the chunk of W H in TMEM,
 //                and A = V / (S + eps) (- 1 for the additive rule), cut the same way; W H is not stored
@@ -18,7 +18,10 @@
 // V is read as it is (FP32, column-major, both half-steps from the one copy): along K it is
 // contiguous for the H-step (rows u) and strided for the W-step (rows i); both arrive by TMA.
 // What bounds it: V's 4 bytes an element from HBM (39.5 us at 8192 x 8192) against
-// 24 MMAs of 128 x npad x 16 a chunk (21.6 us there at r = 64, 43 us at r = 128).
+// 24 MMAs of 128 x npad x 16 a chunk (21.6 us there at r = 64, 43 us at r = 128).  Measured there:
+// kSpEuclid 53 us at r = 64 (the FP32 FMA product: 233), 48 at r = 16; kSpKl 98 at r = 64 and 154 at
+// r = 128, bound by one chunk's chain product -> TMEM load -> quotient -> cut -> TMEM store -> product
+// (the tensor pipe is busy 43-47%); kSpQuality 86 (was ~370), bound by log10 on the FP32 lanes.
 
 enum SpMode { kSpEuclid = 0, kSpKl = 1, kSpKlQuality = 2, kSpQuality = 3, kSpResidual = 4 };
 

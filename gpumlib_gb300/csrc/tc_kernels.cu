@@ -23,10 +23,11 @@
 // as a partial product slot, and the update kernels (one per half-step) sum
 // the slots of a tile in a fixed order, so results are deterministic.
 //
-// Warp roles in the GEMM (192 threads, one CTA per SM):
+// Warp roles in the GEMM (one CTA per SM; gemm_threads):
 //   warp 0      TMA producer (one lane) + TMEM allocation
 //   warp 1      tcgen05.mma issuer (one lane)
 //   warps 2..5  epilogue: tcgen05.ld of their 32-lane TMEM quarter -> partial slot
+//   the rest    the update's prologue, the quality sample, or the Gram
 // Shared memory holds up to 8 stages of (A 16 KB + B N*128 B), 128-byte
 // swizzled as TMA writes them.  TMEM holds two accumulators (N columns
 // each) so the epilogue of one segment overlaps the MMAs of the next.

@@ -17,7 +17,7 @@ the library column-major, as the reference requires (nmf_base.h:92,109).
 Additions beyond the reference: ``Iterate(k)``, ``Residual()`` (FP64
 relative Frobenius residual on the GPU), ``ObjectiveKL()``, an ``eps``
 argument (the reference hard-codes 1e-8) and a ``precision`` argument
-("fp32" = the drop-in path, "bf16" = tensor-core products).
+("fp32" = the drop-in path, FP32 accuracy; "bf16" = BF16 products).
 """
 import ctypes
 

@@ -65,7 +65,8 @@ typedef enum {
 
 /* Arithmetic of the factor products.  The W/H update itself is always FP32. */
 typedef enum {
-    GPUNMF_FP32 = 0,        /* plain FP32 (CUDA cores): the drop-in path         */
+    GPUNMF_FP32 = 0,        /* FP32 accuracy: the drop-in path.  Ranks up to 128: tensor cores, every
+                               operand as three BF16 parts; above: FP32 FMA on the CUDA cores */
     GPUNMF_BF16 = 1         /* BF16 tensor-core products (tcgen05), FP32 accumulate */
 } gpunmf_precision;
 
@@ -238,8 +239,9 @@ gpunmf_status gpunmf_time_iterations(gpunmf_handle h, int iters, int updateW,
 /* Batched small factorisations (Euclidean rule, FP32, ranks 1..32):   */
 /* the counterpart of FacesNMF's grouped training, which runs one NMF  */
 /* object per group in turn (src/examples/FacesNMF/FacesNMFDlg.cpp:    */
-/* 582-656).  All instances run in one persistent, graph-captured      */
-/* launch; each CTA takes whole instances, largest first.              */
+/* 582-656).  All instances' half-steps share their launches, or, for  */
+/* few or very small ones, one persistent, graph-captured launch runs  */
+/* them, a CTA taking whole instances, largest first.                  */
 /* ------------------------------------------------------------------ */
 typedef struct gpunmf_batch gpunmf_batch;
 
@@ -257,7 +259,8 @@ gpunmf_status gpunmf_batch_time(gpunmf_batch *b, int iters, float *ms);
 gpunmf_status gpunmf_batch_get(gpunmf_batch *b, int k, float *W, float *H);
 /* Relative Frobenius residual of every instance (count doubles), FP64 on the GPU. */
 gpunmf_status gpunmf_batch_residuals(gpunmf_batch *b, double *out);
-/* Tile configurations: returns their number; ranks[c] = rank class (4, 8, 16, 32) of config c. */
+/* Tile configurations of the persistent launch (a batch whose instances share their launches ignores
+ * them): returns their number; ranks[c] = rank class (4, 8, 16, 32) of config c. */
 int gpunmf_batch_configs(int *ranks, int cap);
 /* Choose instance k's tile configuration (same rank class), then commit before running. */
 gpunmf_status gpunmf_batch_set_config(gpunmf_batch *b, int k, int cfg);
