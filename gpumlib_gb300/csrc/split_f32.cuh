@@ -153,6 +153,14 @@ __device__ __forceinline__ void two_sum(float2 &s, float2 &c, float2 x) {
     s = t;
 }
 
+// The tensor cores truncate the sum after every step of 16, which leaves a sum of 64 of K low by about half
+// a unit of 2^-23 and one of 128 by about one (measured on positive data: the factors came out 6e-8 and 9e-8
+// off on the mean, 1e-8 to 3e-8 with this).  A sum is scaled by one unit in `halves` of every two chunks.
+// (The batches' sums, of few chunks, are nearer without it: 50 iterations of 768 instances 8.7e-7 against 1.4e-6.)
+__device__ __forceinline__ float truncation(int chunk, int halves) {
+    return (chunk & 1) < halves ? 1.f + 0x1p-23f : 1.f;
+}
+
 // What the update kernel needs of the other factor, from the partials its own update left: this CTA's
 // share of the Gram's entries (four lanes an entry) or of the column / row sums (a warp an entry),
 // by `nt` threads, in a fixed order whatever the number of threads.
@@ -182,8 +190,10 @@ __device__ __forceinline__ void sp_finish_other(const SpParams &p, int et, int n
     } else if constexpr (MODE == kSpKl) {
         const int E = p.npad, lane = et & 31;
         const int e0 = (int)((long long)blockIdx.x * E / gridDim.x), e1 = (int)((long long)(blockIdx.x + 1) * E / gridDim.x);
+        // (in FP64, at most one entry a CTA: a rounded sum moves its whole row of the factor, and the next
+        // iteration moves it again the same way)
         for (int ei = e0 + (et >> 5); ei < e1; ei += nt / 32) {
-            float s = 0.f;
+            double s = 0.0;
             int z = lane;
             for (; z + 7 * 32 < p.sum_count; z += 8 * 32) {
                 float v[8];
@@ -194,7 +204,7 @@ __device__ __forceinline__ void sp_finish_other(const SpParams &p, int et, int n
             }
             for (; z < p.sum_count; z += 32) s += p.sum_partials[(size_t)z * E + ei];
             s = warp_sum(s);
-            if (lane == 0) p.sum_out[ei] = s;
+            if (lane == 0) p.sum_out[ei] = (float)s;
         }
     }
 }
@@ -481,6 +491,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
                 if (!mbar_wait(&d2full[db], dph, p.err, kErrWaitTmemFull, p.wait_limit)) return false;
                 tc_fence_after();
                 constexpr int LD = NC < 16 ? NC : 16;
+                const float up = truncation(dk, 1);
 #pragma unroll
                 for (int g = 0; g < NC / LD; g++)
                     if (c0 + g * LD < p.npad) {
@@ -488,7 +499,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
                         if constexpr (LD == 8) tmem_ld8_sync(tD2 + lane_off + (uint32_t)(db * NPC + c0 + g * LD), v);
                         else tmem_ld16_sync(tD2 + lane_off + (uint32_t)(db * NPC + c0 + g * LD), v);
 #pragma unroll
-                        for (int c = 0; c < LD; c++) acc[g * LD + c] += v[c];
+                        for (int c = 0; c < LD; c++) acc[g * LD + c] = fmaf(v[c], up, acc[g * LD + c]);
                     }
                 tc_fence_before();
                 __syncwarp();
@@ -572,13 +583,14 @@ __global__ void __launch_bounds__(kSpThreads, 1)
                 // (Markstein), which a division in range rounds like the operator but for rare last
                 // bits, without its branch; a warp with any other division takes the operator
                 const float less = p.minus_one ? 1.f : 0.f;
+                const float up = truncation(kk, p.npad < 32 ? 0 : p.npad < 96 ? 1 : 2);
 #pragma unroll
                 for (int h = 0; h < 16; h += 8) {
                     float q[8], dmax = 0.f;
                     bool fine = true;
 #pragma unroll
                     for (int c = 0; c < 8; c++) {
-                        const float d = s[h + c] + p.eps, y = rcp_approx(d), a = v[h + c] * y;
+                        const float d = fmaf(s[h + c], up, p.eps), y = rcp_approx(d), a = v[h + c] * y;
                         q[c] = fmaf(fmaf(-a, d, v[h + c]), y, a);
                         dmax = fmaxf(dmax, fabsf(d));
                         fine = fine && fabsf(q[c]) < 1e38f;
@@ -586,8 +598,8 @@ __global__ void __launch_bounds__(kSpThreads, 1)
                     if (__any_sync(0xffffffffu, !fine || dmax > 8e37f || h + 8 > klim)) {
 #pragma unroll
                         for (int c = 0; c < 8; c += 2) {  // beyond K: 0 (not 0 / eps)
-                            const float x = h + c < klim ? v[h + c] / (s[h + c] + p.eps) - less : 0.f;
-                            const float y = h + c + 1 < klim ? v[h + c + 1] / (s[h + c + 1] + p.eps) - less : 0.f;
+                            const float x = h + c < klim ? v[h + c] / fmaf(s[h + c], up, p.eps) - less : 0.f;
+                            const float y = h + c + 1 < klim ? v[h + c + 1] / fmaf(s[h + c + 1], up, p.eps) - less : 0.f;
                             uint32_t a[3], b[3];
                             cut3(x, a[0], a[1], a[2]);
                             cut3(y, b[0], b[1], b[2]);
