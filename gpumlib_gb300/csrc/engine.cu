@@ -737,9 +737,9 @@ gpunmf_status gpunmf_residual_fp64(gpunmf_handle h, double *out) {
     job_residual_ready(h);
     TRY_STATUS(job_residual(h, h->d_scalar));
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(h->h_scalar(), h->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, s));
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(s));
-    *out = h->h_scalar()[0];
-    return tc_check(h);
+    const gpunmf_status st = tc_check_sync(h);
+    if (st == GPUNMF_OK || st == GPUNMF_ERR_TIMEOUT) *out = h->h_scalar()[0];
+    return st;
 }
 
 gpunmf_status gpunmf_objective_kl_fp64(gpunmf_handle h, double *out) {
@@ -765,16 +765,14 @@ gpunmf_status gpunmf_get_w(gpunmf_handle h, float *W) {
     CHECK_HANDLE(h);
     if (!W) return GPUNMF_ERR_INVALID;
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(W, h->W, sizeof(float) * (size_t)h->n * h->r, cudaMemcpyDeviceToHost, h->stream));
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return tc_check(h);
+    return tc_check_sync(h);
 }
 
 gpunmf_status gpunmf_get_h(gpunmf_handle h, float *H) {
     CHECK_HANDLE(h);
     if (!H) return GPUNMF_ERR_INVALID;
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(H, h->H, sizeof(float) * (size_t)h->r * h->m, cudaMemcpyDeviceToHost, h->stream));
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return tc_check(h);
+    return tc_check_sync(h);
 }
 
 gpunmf_status gpunmf_get_wh(gpunmf_handle h, float *WH) {
@@ -795,8 +793,7 @@ gpunmf_status gpunmf_device_factors(gpunmf_handle h, float **dW, float **dH) {
 
 gpunmf_status gpunmf_synchronize(gpunmf_handle h) {
     CHECK_HANDLE(h);
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return tc_check(h);
+    return tc_check_sync(h);
 }
 
 gpunmf_status gpunmf_info(gpunmf_handle h, int *rule, int *n, int *m, int *r, int *precision, float *eps) {
@@ -842,7 +839,7 @@ gpunmf_status gpunmf_time_iterations(gpunmf_handle h, int iters, int updateW, fl
         return GPUNMF_ERR_CUDA;
     }
     if (st != GPUNMF_OK) return st;
-    st = tc_check(h);
+    st = tc_check_sync(h);
     if (st != GPUNMF_OK) return st;
     if (total_ms) *total_ms = ms;
     if (kernel_ms) {

@@ -32,8 +32,9 @@ struct gpunmf_job {
     size_t red_cap = 0;
     float *d_quality = nullptr;
     double *d_scalar = nullptr;
-    unsigned char *h_pinned = nullptr;        // 64 pinned bytes: quality (float) at 0, scalar (double) at 8
+    unsigned char *h_pinned = nullptr;        // 64 pinned bytes: quality (float) at 0, scalar (double) at 8, errors (2 ints) at 16
     float *h_quality() { return reinterpret_cast<float *>(h_pinned); }
+    int *h_errors() { return reinterpret_cast<int *>(h_pinned + 16); }
     double *h_scalar() { return reinterpret_cast<double *>(h_pinned + 8); }
 
     // quality bookkeeping (src/algorithms/nmf/nmf_base.h:49-53)
@@ -101,7 +102,7 @@ gpunmf_status tc_quality(gpunmf_job *j);
 // fused Euclidean and KL jobs: the next H-step launch samples the quality itself (it also records the
 // job's quality event); false where it cannot
 bool tc_quality_fold(gpunmf_job *j);
-gpunmf_status tc_check(gpunmf_job *j);    // reads the kernels' error word (after a sync)
+gpunmf_status tc_check_sync(gpunmf_job *j);  // waits for the job's stream and reads the kernels' error words
 void tc_set_wait_limit(gpunmf_job *j, long long cycles);  // <= 0: the default (about 2 s)
 gpunmf_status tc_inject_missing_arrival(gpunmf_job *j);
 void tc_set_grid_limit(int ctas);         // CTAs per launch of jobs created later (0: one per SM)
