@@ -2422,12 +2422,9 @@ __global__ void __launch_bounds__(kKlThreads)
                 }
                 // this part's 32 columns: 64-column box part / 2, 16-byte chunks 4 (part & 1) ..
                 const unsigned char *vt = sV(vi) + (part >> 1) * (kKlVBytes / 2);
-                uint4 vraw[4];
+                float4 vraw[4];
 #pragma unroll
-                for (int cc = 0; cc < 4; cc++) vraw[cc] = *reinterpret_cast<const uint4 *>(vt + sw128(row, (part & 1) * 4 + cc));
-                // the V stage is read (the arrive orders the loads before the producer's refill)
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&vempty[vi]);
+                for (int cc = 0; cc < 4; cc++) vraw[cc] = lds128_stage(smem_u32(vt) + sw128(row, (part & 1) * 4 + cc));
                 if constexpr (QF) {
                     tmem_ld16_sync(ta, *reinterpret_cast<float (*)[16]>(&sv[0]));
                     tmem_ld16_sync(ta + 16, *reinterpret_cast<float (*)[16]>(&sv[16]));
@@ -2453,8 +2450,13 @@ __global__ void __launch_bounds__(kKlThreads)
                 tmem_st16(ta, rr);
                 tmem_st_wait();
                 tc_fence_before();
+                // The V stage goes back only here, when every value read of it has been used: an arrive right
+                // after the loads does not wait for their data, so the producer could refill the stage first.
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&rfull[di]);
+                if (lane == 0) {
+                    mbar_arrive(&rfull[di]);
+                    mbar_arrive(&vempty[vi]);
+                }
                 if constexpr (QF) {
                     // the sample, behind the chain: the second product has its R already.  (As a launch of
                     // its own it streamed V and formed W H again: 45 us an iteration of 140 at 16384 x
