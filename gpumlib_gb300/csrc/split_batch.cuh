@@ -114,12 +114,16 @@ __global__ void __launch_bounds__(kSpbThreads, 1) spb_kernel(SpbParams p) {
         if (lane == 0 && nblk > 0) {
             const uint64_t vpol = l2_policy_evict_first();
             SpbCursor cv(p, first), cf(p, first);
-            int vj = 0, vs = 0, fj = 0, fs = 0;
+            int vj = 0, vs = 0, fj = 0, fs = 0, vinst = -1, finst = -1;
             uint32_t vph = 0, fph = 0, par_v = 0, par_f = 0;
             auto load_v = [&] {
                 mbar_arrive_expect_tx(&vfull[vs], (uint32_t)kSpVBytes);
                 unsigned char *dst = sVr + vs * kSpVBytes;
                 const CUtensorMap *tm = p.mapV + cv.cur.inst;
+                if (cv.cur.inst != vinst) {
+                    vinst = cv.cur.inst;
+                    tma_acquire_desc(tm);
+                }
                 if (K_CONTIG) {
                     tma_load_2d_hint(dst, tm, cv.k * kSpChunk, cv.cur.row * kTileM, &vfull[vs], vpol);
                     tma_load_2d_hint(dst + kSpVBytes / 2, tm, cv.k * kSpChunk + 32, cv.cur.row * kTileM, &vfull[vs], vpol);
@@ -140,7 +144,11 @@ __global__ void __launch_bounds__(kSpbThreads, 1) spb_kernel(SpbParams p) {
                 bool moved = false;
                 if (fj < nblk && (fj < kSpbStages || mbar_test(&fempty[fs], fph ^ 1))) {
                     mbar_arrive_expect_tx(&ffull[fs], (uint32_t)kSpFBox);
-                    tma_load_3d(sFr + fs * kSpFBox, p.mapF + cf.cur.inst, 0, cf.k * kSpChunk, 0, &ffull[fs]);
+                    if (cf.cur.inst != finst) {
+                        finst = cf.cur.inst;
+                        tma_acquire_desc(p.mapF + finst);
+                    }
+                    tma_load_3d(sFr + fs * kSpFBox, p.mapF + finst, 0, cf.k * kSpChunk, 0, &ffull[fs]);
                     par_f = (par_f & ~(1u << fs)) | (fph << fs);
                     ring_next(fs, fph, kSpbStages);
                     fj++;

@@ -177,6 +177,12 @@ __device__ __forceinline__ float lds32_stage(uint32_t addr) {
     return v;
 }
 
+// Before the first use of a tensor map that lies in global memory, by the thread that uses it: the maps are
+// cached, and what a copy wrote over an earlier map at the same address is not seen without it.
+__device__ __forceinline__ void tma_acquire_desc(const CUtensorMap *tm) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(tm)) : "memory");
+}
+
 // ---------------------------------------------------------------- programmatic dependent launch
 // Wait until the grids this one depends on have completed and their writes are visible.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
