@@ -14,6 +14,7 @@
 struct SpbInst {
     int n, m, r, npad;
     long long ldv;                          // column stride of V
+    float low_h, low_w;                     // what the numerators are low by (sp_low_sum)
     const float *V;
     float *W, *H;
     __nv_bfloat16 *Ws, *Hs;                 // three parts, [part][row][npad]
@@ -354,6 +355,7 @@ __global__ void __launch_bounds__(kSpbUpdThreads, 4) spb_update_kernel(SpbUpdPar
     u.update = p.update;
     u.V = d.V;
     u.ldv = d.ldv;
+    u.low = p.is_w ? d.low_w : d.low_h;
     u.F = p.is_w ? d.H : d.W;
     if (d.npad == 16) update_rows<16, kSpbRows, kSpbUpdThreads>(u, b.row0, b.row0 / kSpbRows, sm);
     else update_rows<32, kSpbRows, kSpbUpdThreads>(u, b.row0, b.row0 / kSpbRows, sm);
@@ -496,6 +498,7 @@ gpunmf_status spb_create(const std::vector<SpbShape> &shapes, float eps, cudaStr
             SpbInst &d = insts[i];
             const size_t np = npad_of(q.r);
             d.n = q.n; d.m = q.m; d.r = q.r; d.npad = (int)np; d.ldv = (q.n + 3) / 4 * 4;
+            d.low_h = sp_low_sum(q.n); d.low_w = sp_low_sum(q.m);
             d.V = q.V; d.W = q.W; d.H = q.H;
             a.get(&d.Ws, 3 * (size_t)q.n * np);
             a.get(&d.Hs, 3 * (size_t)q.m * np);

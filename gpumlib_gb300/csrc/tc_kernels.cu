@@ -1583,6 +1583,9 @@ struct UpdParams {
     const float *V, *F;       // FP32 products: V (column-major, stride ldv) and the other factor, for plain_sum
     long long ldv;
     int K;
+    const float2 *checks;     // FP32 products: what the slots' rows are low by and their size (SpParams), or (null)
+    float low;                // the fraction expected (sp_low_sum)
+    float *row_sums;          // [cols] sums of X's rows, for the next product's check sums (or null)
     int slot0, slots;         // batches (slot_ptr null): the tile's slots, numbered on
 };
 
@@ -1594,6 +1597,63 @@ __device__ __noinline__ float plain_sum(int is_w, const float *V, long long ldv,
         s = is_w ? fmaf(V[(long long)k * ldv + row], F[(long long)k * r + a], s)
                  : fmaf(V[(long long)row * ldv + k], F[(long long)a * K + k], s);
     return s;
+}
+
+// What to add to a row's numerators, as a fraction of each one's size: d, by how much the checked sums are
+// low together, over the sum of their sizes; without any, what is expected.  (No cut of the tensor cores
+// comes near 2^-18: a sum that is off by more, infinite or NaN says nothing.)
+__device__ __forceinline__ float low_fraction(float d, float size, float expected) {
+    return size == 0.f ? expected : fabsf(d) <= size * 0x1p-18f ? __fdividef(d, size) : 0.f;
+}
+
+// The slots' checks of ROWS rows, summed by NT threads: neighbours take neighbouring rows (so that a warp's loads are
+// whole sectors), ROWS threads a quarter of a slot.  The first CP quarters of a thread are loaded by begin,
+// with the kernel's other first loads; finish leaves part sums in shared memory, fraction adds a row's up.
+template <int ROWS, int NT, int CP>
+struct RowChecks {
+    static constexpr int NK = NT / ROWS, PARTS = ROWS < 32 ? NT / 32 : NK;
+    const float2 *checks;
+    const int *list;
+    int s0, n, id[CP];  // n: quarters of slots
+    float2 v[CP];
+    // (the slot lists do not change: read before the wait for the kernel that fills the slots)
+    __device__ __forceinline__ RowChecks(const float2 *c, const int *l, int s0_, int s1, int tid) : checks(c), list(l), s0(s0_), n(4 * (s1 - s0_)) {
+#pragma unroll
+        for (int i = 0; i < CP; i++) id[i] = checks && tid / ROWS + i * NK < n ? list[s0 + (tid / ROWS + i * NK) / 4] : -1;
+    }
+    __device__ __forceinline__ float2 at(int slot, int k, int row) const {
+        return slot < 0 ? make_float2(0.f, 0.f) : __ldcg(checks + ((size_t)slot * 4 + k % 4) * 128 + row);
+    }
+    __device__ __forceinline__ void begin(int tid, int lrow0) {
+#pragma unroll
+        for (int i = 0; i < CP; i++) v[i] = at(id[i], tid / ROWS + i * NK, lrow0 + tid % ROWS);
+    }
+    __device__ __forceinline__ void finish(int tid, int lrow0, float2 (&sums)[PARTS][ROWS]) const {
+        float2 c = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < CP; i++) c = make_float2(c.x + v[i].x, c.y + v[i].y);
+        for (int k = tid / ROWS + CP * NK; k < n; k += NK) {
+            const float2 w = at(list[s0 + k / 4], k, lrow0 + tid % ROWS);
+            c = make_float2(c.x + w.x, c.y + w.y);
+        }
+#pragma unroll
+        for (int o = ROWS; o < 32; o <<= 1) {
+            c.x += __shfl_xor_sync(0xffffffffu, c.x, o);
+            c.y += __shfl_xor_sync(0xffffffffu, c.y, o);
+        }
+        if (ROWS >= 32 || (tid & 31) < ROWS) sums[ROWS < 32 ? tid / 32 : tid / ROWS][tid % ROWS] = c;
+    }
+    __device__ __forceinline__ static float fraction(const float2 (&sums)[PARTS][ROWS], int row, float expected) {
+        float2 c = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < PARTS; k++) c = make_float2(c.x + sums[k][row].x, c.y + sums[k][row].y);
+        return low_fraction(c.x, c.y, expected);
+    }
+};
+
+// x q + e, rounded once, for an e that is small beside y = x q; an infinity or NaN stays what y is
+__device__ __forceinline__ float plus_product(float x, float q, float y, float e) {
+    return fabsf(e) < __int_as_float(0x7F800000) ? fmaf(x, q, e) : y;
 }
 
 // Rows per CTA and its threads.  Up to rank 64: 16 rows, 256 threads; several CTAs of an SM overlap their
@@ -1644,8 +1704,13 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
     }
 #pragma unroll
     for (int q = 0; q < kIds; q++) ids[q] = p.slot_ptr && p.update ? p.slot_list[min(s0 + q, s1 - 1)] : min(s0 + q, s1 - 1);
+    const int ga = tid & 15, gc = tid >> 4;
+    const bool checks = p.checks && p.update;
+    RowChecks<ROWS, NT, ROWS == 64 ? 2 : 4> rc(checks ? p.checks : nullptr, p.slot_list, s0, s1, tid);
+    __shared__ float2 row_checks[decltype(rc)::PARTS][ROWS];
     griddep_wait();  // the GEMM's partial slots and Gram are complete
     griddep_launch_dependents();
+    rc.begin(tid, lrow0);
     // the old rows, zero outside r and ncol; a thread issues up to sixteen loads before it stores
     constexpr int XL = RP * ROWS / NT, XB = XL < 16 ? XL : 16;
 #pragma unroll 1
@@ -1673,6 +1738,7 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
         for (int j = 0; j < XB; j++)
             if (at[j] >= 0) Xs[at[j]] = xv[j];
     }
+    if (checks) rc.finish(tid, lrow0, row_checks);
     if (p.update) {
         // G (RP x RP; the rows of X beyond r are zero)
         constexpr int G4 = RP * RP / 4;
@@ -1730,7 +1796,6 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
         }
     }
     __syncthreads();
-    const int ga = tid & 15, gc = tid >> 4;
     if (p.update) {
         float den[TA][RT];
 #pragma unroll
@@ -1747,6 +1812,9 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
 #pragma unroll
                 for (int j = 0; j < RT; j++) den[i][j] = fmaf(g[i], xb[j], den[i][j]);
         }
+        float low[RT];
+#pragma unroll
+        for (int j = 0; j < RT; j++) low[j] = checks ? rc.fraction(row_checks, gc * RT + j, p.low) : p.low;
 #pragma unroll
         for (int i = 0; i < TA; i++) {
             const int a = upd_col<TA>(ga, i);
@@ -1757,11 +1825,14 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
                 const float nv = *at;
                 float x = Xs[a * LDX + c];
                 if (a < r && c < ncol) {  // outside stays 0 (the additive step has no eps)
+                    // (FP32 products: the rounding there is takes the fraction in)
                     if (p.additive) {
-                        x = x + (x / den[i][j]) * (nv - den[i][j]);
+                        const float step = nv - den[i][j];
+                        x = x + (x / den[i][j]) * (p.Xs && low[j] != 0.f ? fmaf(fabsf(nv), low[j], step) : step);
                         x = x < 0.f ? 0.f : x;
                     } else {
-                        x *= nv / (den[i][j] + p.eps);
+                        const float q = nv / (den[i][j] + p.eps), y = x * q;
+                        x = p.Xs ? plus_product(x, q, y, fabsf(y) * low[j]) : y;
                     }
                 } else {
                     x = 0.f;
@@ -1802,6 +1873,14 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
             Ns[c * LDN + a] = Xs[a * LDX + c];
         }
         __syncthreads();
+    }
+    if (p.row_sums) {
+        constexpr int G = NT / ROWS;
+        float z = 0.f;
+        for (int a = tid % G; a < RP; a += G) z += Ns[tid / G * LDN + a];
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+        if (tid % G == 0 && tid / G < ncol) p.row_sums[c0 + tid / G] = z;
     }
     // partial Gram of the new rows (those outside ncol are zero), 256 threads with a TA x TA block each.
     // BF16 jobs: one for every 16 rows (a sum over more rows at once would round differently, and the
@@ -2575,6 +2654,9 @@ struct KlUpdParams {
     int update;
     int additive;        // 1: X = max(0, X + (X / max(sum, eps)) (num - sum)); 2: num has the - sum already
     long long part;      // FP32 products (Xb null): Xr holds the three parts of X, this far apart
+    const float2 *checks;  // FP32 products: what the slots' rows are low by (UpdParams)
+    float low, s_low;    // the fractions that a numerator (without a check) and S are expected to be low by
+    float *row_sums;     // [cols] sums of X's rows (FP32 products)
 };
 
 // COLS columns of H (rows of W) per CTA: 8 for the H-step (its m is the smaller side: more CTAs),
@@ -2588,13 +2670,18 @@ __global__ void __launch_bounds__(kUpdThreads) tc_kl_update_kernel(KlUpdParams p
     constexpr int TOT = RP * COLS;  // 128 (r <= 16 in the H-step) up to 2048 elements
     constexpr int XL = (TOT + kUpdThreads - 1) / kUpdThreads;
     __shared__ float Xs[RP * LDX];
-    __shared__ float sumS[RP], sumR[RP];
+    __shared__ float sumS[RP], sumR[RP], rowD[COLS];
     const int tid = threadIdx.x;
     const int c0 = blockIdx.x * COLS;
     const int ncol = min(COLS, p.cols - c0);
     const int r = p.r;
+    const bool checks = p.checks && p.update;
+    const int *sp = checks ? p.slot_ptr + c0 / 128 : nullptr;
+    RowChecks<COLS, kUpdThreads, COLS == 8 ? 2 : 4> rc(checks ? p.checks : nullptr, p.slot_list, sp ? sp[0] : 0, sp ? sp[1] : 0, tid);
+    __shared__ float2 row_checks[decltype(rc)::PARTS][COLS];
     griddep_wait();
     griddep_launch_dependents();
+    rc.begin(tid, c0 % 128);
 #pragma unroll
     for (int j = 0; j < XL; j++) {  // the old rows, zero beyond r and beyond the last column
         const int k = tid + j * kUpdThreads;
@@ -2612,6 +2699,7 @@ __global__ void __launch_bounds__(kUpdThreads) tc_kl_update_kernel(KlUpdParams p
         sumS[tid] = p.update ? fmaxf(sraw, p.eps) : 1.f;
         sumR[tid] = sraw;
     }
+    if (checks) rc.finish(tid, c0 % 128, row_checks);
     float acc[XL];
 #pragma unroll
     for (int j = 0; j < XL; j++) acc[j] = 0.f;
@@ -2660,17 +2748,25 @@ __global__ void __launch_bounds__(kUpdThreads) tc_kl_update_kernel(KlUpdParams p
         }
     }
     __syncthreads();
+    if (checks) {
+        if (tid < COLS) rowD[tid] = rc.fraction(row_checks, tid, p.low);
+        __syncthreads();
+    }
     if (p.update) {
 #pragma unroll
         for (int j = 0; j < XL; j++) {
             const int k = tid + j * kUpdThreads, c = k / RP, a = k % RP;
             if (a < r && c < ncol) {
                 float x = Xs[a * LDX + c];
+                // (FP32 products: S low by s_low raises every quotient, and so the numerator, by it)
                 if (p.additive) {
-                    x = x + (x / sumS[a]) * (p.additive == 1 ? acc[j] - sumR[a] : acc[j]);
+                    const float q = x / sumS[a], num = p.additive == 1 ? acc[j] - sumR[a] : acc[j];
+                    if (p.checks) x = x + plus_product(q, num, q * num, q * (rowD[c] * fabsf(num) - p.s_low * (num + sumR[a])));
+                    else x = x + q * num;
                     x = x < 0.f ? 0.f : x;
                 } else {
-                    x *= (acc[j] / sumS[a]);
+                    const float q = acc[j] / sumS[a], y = x * q;
+                    x = p.checks ? plus_product(x, q, y, fabsf(y) * (rowD[c] - p.s_low)) : y;
                 }
                 Xs[a * LDX + c] = x;
             }
@@ -2699,6 +2795,15 @@ __global__ void __launch_bounds__(kUpdThreads) tc_kl_update_kernel(KlUpdParams p
             if (p.Xb) p.Xr[(long long)(c0 + c) * p.ldr + a] = __float2bfloat16_rn(x);
             else store_cut(p.Xr + (long long)(c0 + c) * p.ldr + a, p.part, x);
         }
+    }
+    if (p.row_sums) {
+        constexpr int T = kUpdThreads / COLS;
+        const int c = tid / T;
+        float z = 0.f;
+        for (int a = tid % T; a < r; a += T) z += Xs[a * LDX + c];
+#pragma unroll
+        for (int o = 1; o < T; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+        if (tid % T == 0 && c < ncol) p.row_sums[c0 + c] = z;
     }
     if (tid < RP) {
         float sacc = 0.f;
