@@ -454,7 +454,7 @@ __global__ void batch_residual_kernel(const BatchInst *__restrict__ insts, int c
     }
     num = block_sum(num, red);
     den = block_sum(den, red);
-    if (threadIdx.x == 0) out[k] = den > 0.0 ? sqrt(num / den) : 0.0;
+    if (threadIdx.x == 0) out[k] = relative_residual(num, den);
 }
 
 }  // namespace gpunmf

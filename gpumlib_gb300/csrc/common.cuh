@@ -56,6 +56,9 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
     return out;
 }
 
+// sqrt(num / den) of a relative residual's sums: 0 for a zero matrix, NaN where a sum is
+__device__ __forceinline__ double relative_residual(double num, double den) { return den == 0.0 ? 0.0 : sqrt(num / den); }
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace gpunmf

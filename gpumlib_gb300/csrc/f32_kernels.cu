@@ -684,7 +684,7 @@ __global__ void finalize_kernel(const double *__restrict__ partial, int count, i
             if (out_f) out_f[0] = (float)s0;
             if (out_d) out_d[0] = s0;
         } else {
-            double rr = s1 > 0.0 ? sqrt(s0 / s1) : 0.0;
+            double rr = relative_residual(s0, s1);
             if (out_d) out_d[0] = rr;
             if (out_f) out_f[0] = (float)rr;
         }

@@ -493,6 +493,7 @@ __global__ void __launch_bounds__(NPC == 32 && MODE == kSpEuclid ? 768 : kSpThre
         int vs = 0, rb = 0, d1 = 0, db = 0, kk = kc0, t = t0, seg = 0, dk = kc0, dseg = 0;
         uint32_t vph = 0, rph = 0, d1ph = 0, dph = 0;
         float2 qs = both(0.f), qc = qs, ws = qs, wc = qs;  // two-term sums
+        double far_a = 0.0, far_b = 0.0;  // the residual's sums of what FP32 squares do not hold
         float acc[kReduce ? 1 : NC];
         if constexpr (!kReduce) {
 #pragma unroll
@@ -663,11 +664,28 @@ __global__ void __launch_bounds__(NPC == 32 && MODE == kSpEuclid ? 768 : kSpThre
             } else if constexpr (MODE == kSpQuality) {
                 sample(v, s, klim);
             } else {
-                // (v - s)^2 and v^2 with what FP32 drops of them (zeros beyond the last row and K)
+                // (v - s)^2 and v^2 with what FP32 drops of them (zeros beyond the last row and K).  Where the
+                // squares leave FP32's range (a value above 2^50, an infinity, or all of the sixteen below
+                // 2^-40) they are formed in FP64.
                 if (klim < 16) {
 #pragma unroll
                     for (int c = 0; c < 16; c++)
                         if (c >= klim) v[c] = s[c] = 0.f;
+                }
+                float most = 0.f;
+#pragma unroll
+                for (int c = 0; c < 16; c++) most = fmaxf(most, fmaxf(fabsf(v[c]), fabsf(s[c])));
+                if (__any_sync(0xffffffffu, most != 0.f && !(most >= 0x1p-40f && most <= 0x1p50f))) {
+                    if (!(most >= 0x1p-40f && most <= 0x1p50f)) {
+#pragma unroll
+                        for (int c = 0; c < 16; c++) {
+                            const double d = (double)v[c] - (double)s[c];
+                            far_a += d * d;
+                            far_b += (double)v[c] * (double)v[c];
+                            v[c] = s[c] = 0.f;
+                        }
+                    }
+                    __syncwarp();
                 }
 #pragma unroll
                 for (int c = 0; c < 16; c += 2) {
@@ -729,6 +747,10 @@ __global__ void __launch_bounds__(NPC == 32 && MODE == kSpEuclid ? 768 : kSpThre
         if constexpr (kSum) {
             double a = ((double)qs.x + (double)qc.x) + ((double)qs.y + (double)qc.y);
             double b = ((double)ws.x + (double)wc.x) + ((double)ws.y + (double)wc.y);
+            if (MODE == kSpResidual) {
+                a += far_a;
+                b += far_b;
+            }
             a = warp_sum(a);
             if (MODE == kSpResidual) b = warp_sum(b);
             if (lane == 0) {
@@ -768,7 +790,7 @@ __global__ void __launch_bounds__(NPC == 32 && MODE == kSpEuclid ? 768 : kSpThre
             if constexpr (kTerms == 2) b = warp_sum(b);
             if (lane == 0) {
                 if constexpr (kTerms == 2) {
-                    p.rout[0] = b > 0.0 ? sqrt(a / b) : 0.0;
+                    p.rout[0] = relative_residual(a, b);
                 } else {
                     p.qout[0] = (float)a;
                     if (p.qout_host) {
