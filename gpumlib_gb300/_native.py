@@ -43,6 +43,7 @@ SIGNATURES = [
     ("gpunmf_get_wh", ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
     ("gpunmf_device_factors", ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p),
                                               ctypes.POINTER(ctypes.c_void_p)]),
+    ("gpunmf_factors_changed", ctypes.c_int, [ctypes.c_void_p]),
     ("gpunmf_synchronize", ctypes.c_int, [ctypes.c_void_p]),
     ("gpunmf_info", ctypes.c_int, [ctypes.c_void_p, c_int_p, c_int_p, c_int_p, c_int_p, c_int_p, c_float_p]),
     ("gpunmf_footprint_bytes", ctypes.c_size_t, [ctypes.c_int] * 5),

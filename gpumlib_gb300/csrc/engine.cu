@@ -485,7 +485,17 @@ static gpunmf_status iterate_kl_f32(gpunmf_job *j, bool updateW) {
     return GPUNMF_OK;
 }
 
+// Jobs keep copies and sums of their factors (BF16 copies, parts, Gram partials): made again where a caller may have
+// written the factors through their device pointers.
+static gpunmf_status job_refresh(gpunmf_job *j) {
+    if (!j->factors_changed) return GPUNMF_OK;
+    j->factors_changed = false;
+    if (j->tc) return tc_refresh(j);
+    return j->sp ? sp_refresh(j) : GPUNMF_OK;
+}
+
 static gpunmf_status job_iterate(gpunmf_job *j, int iters, bool updateW) {
+    if (iters > 0) TRY_STATUS(job_refresh(j));
     for (int it = 0; it < iters; it++) {
         gpunmf_status st;
         if (j->precision == GPUNMF_BF16)
@@ -734,6 +744,7 @@ gpunmf_status gpunmf_residual_fp64(gpunmf_handle h, double *out) {
     CHECK_HANDLE(h);
     if (!out) return GPUNMF_ERR_INVALID;
     cudaStream_t s = h->stream;
+    TRY_STATUS(job_refresh(h));
     job_residual_ready(h);
     TRY_STATUS(job_residual(h, h->d_scalar));
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(h->h_scalar(), h->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -788,6 +799,12 @@ gpunmf_status gpunmf_device_factors(gpunmf_handle h, float **dW, float **dH) {
     CHECK_HANDLE(h);
     if (dW) *dW = h->W;
     if (dH) *dH = h->H;
+    return GPUNMF_OK;
+}
+
+gpunmf_status gpunmf_factors_changed(gpunmf_handle h) {
+    CHECK_HANDLE(h);
+    h->factors_changed = true;
     return GPUNMF_OK;
 }
 

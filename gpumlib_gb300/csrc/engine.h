@@ -51,6 +51,8 @@ struct gpunmf_job {
     int timed_launches = 0;
     std::vector<cudaEvent_t> tev;
 
+    bool factors_changed = false;  // the factors may have been written from outside since the last call
+
     TcState *tc = nullptr;
     SpState *sp = nullptr;  // FP32 jobs of rank <= 128; BF16 jobs of such ranks for their residual
 
@@ -93,6 +95,7 @@ gpunmf_status tc_create(gpunmf_job *j);
 // after V/W/H are uploaded; or, with v_src (V in host memory the device can read), after W/H are:
 // then the BF16 conversion reads V from there and also writes the job's FP32 V
 gpunmf_status tc_prepare(gpunmf_job *j, const float *v_src = nullptr);
+gpunmf_status tc_refresh(gpunmf_job *j);  // after the factors on the device have changed
 gpunmf_status tc_iterate(gpunmf_job *j, bool updateW);
 // quality of the current factors on the tensor cores (BF16 jobs with npad <= 128)
 bool tc_quality_ready(const gpunmf_job *j);
@@ -114,6 +117,7 @@ bool sp_supported(int n, int m, int r);
 size_t sp_footprint(int rule, int n, int m, int r, bool residual_only);
 gpunmf_status sp_create(gpunmf_job *j, bool residual_only);
 gpunmf_status sp_prepare(gpunmf_job *j, bool residual_only);  // after V, W, H are on the device
+gpunmf_status sp_refresh(gpunmf_job *j);  // after the factors on the device have changed
 gpunmf_status sp_iterate(gpunmf_job *j, bool updateW);
 gpunmf_status sp_quality(gpunmf_job *j);
 bool sp_quality_writes_host(const gpunmf_job *j);

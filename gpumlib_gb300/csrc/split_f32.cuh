@@ -1219,6 +1219,15 @@ static cudaError_t sp_cut_factors(gpunmf_job *j) {
     return cudaGetLastError();
 }
 
+// What an FP32 job keeps beside its factors, made of them: the parts of both, and the row sums and Gram / sum partials
+// of W (of H too for the rule that keeps it).
+gpunmf_status sp_refresh(gpunmf_job *j) {
+    GPUNMF_CUDA_TRY(sp_cut_factors(j));
+    GPUNMF_CUDA_TRY(sp_update(j, true, 0));
+    if (j->rule == GPUNMF_ADDITIVE_EUCLIDEAN_FIXED_H) GPUNMF_CUDA_TRY(sp_update(j, false, 0));
+    return GPUNMF_OK;
+}
+
 gpunmf_status sp_prepare(gpunmf_job *j, bool residual_only) {
     SpState *t = j->sp;
     if (t->Vp) {
@@ -1226,12 +1235,7 @@ gpunmf_status sp_prepare(gpunmf_job *j, bool residual_only) {
             j->V, j->n, j->m, t->Vp, (j->n + 3) / 4 * 4);
         GPUNMF_CUDA_TRY(cudaGetLastError());
     }
-    if (residual_only) return GPUNMF_OK;
-    GPUNMF_CUDA_TRY(sp_cut_factors(j));
-    // the Gram / sum partials of the initial W, and of H for the rule that keeps it
-    GPUNMF_CUDA_TRY(sp_update(j, true, 0));
-    if (j->rule == GPUNMF_ADDITIVE_EUCLIDEAN_FIXED_H) GPUNMF_CUDA_TRY(sp_update(j, false, 0));
-    return GPUNMF_OK;
+    return residual_only ? GPUNMF_OK : sp_refresh(j);
 }
 
 bool sp_quality_writes_host(const gpunmf_job *j) { return j->sp->gq.p.qout_host != nullptr; }

@@ -3768,6 +3768,14 @@ gpunmf_status tc_prepare(gpunmf_job *j, const float *v_src) {
     // from the job's V, or straight from the caller's matrix (which also fills the job's V)
     convert_v_kernel<<<dim3(t->npr / 64, t->mpr / 64), 256, 0, s>>>(v_src ? v_src : j->V, j->n, j->m, t->npr, t->mpr,
                                                                     t->Vb, t->Vbt, v_src ? j->V : nullptr);
+    GPUNMF_CUDA_TRY(cudaGetLastError());
+    return tc_refresh(j);
+}
+
+// What a BF16 job keeps beside its factors, made of them
+gpunmf_status tc_refresh(gpunmf_job *j) {
+    TcState *t = j->tc;
+    cudaStream_t s = j->stream;
     convert_w_kernel<<<std::min(1024, ceil_div((long long)j->n * j->r, 256)), 256, 0, s>>>(j->W, j->n, j->r,
                                                                                           t->Wb, t->ldw);
     convert_h_kernel<<<std::min(1024, ceil_div((long long)j->r * j->m, 256)), 256, 0, s>>>(j->H, j->r, j->m,

@@ -198,8 +198,15 @@ gpunmf_status gpunmf_get_w(gpunmf_handle h, float *W);
 gpunmf_status gpunmf_get_h(gpunmf_handle h, float *H);
 gpunmf_status gpunmf_get_wh(gpunmf_handle h, float *WH);
 
-/* Device pointers of the job's FP32 factors (valid until destroy). */
+/* Device pointers of the job's FP32 factors (valid until destroy).  A job also keeps copies and sums of
+ * its factors, which its iterations read; a caller that writes through the pointers says so with
+ * gpunmf_factors_changed before the job's next call, and its writes must come before that call in the
+ * order of the job's stream.  (FP32 jobs of ranks above 128 read the factors themselves; the call does
+ * nothing there.) */
 gpunmf_status gpunmf_device_factors(gpunmf_handle h, float **dW, float **dH);
+/* The factors have been written through their device pointers: the job's next iteration or residual
+ * first makes its copies and sums of them again. */
+gpunmf_status gpunmf_factors_changed(gpunmf_handle h);
 
 /* Wait for the job's queued work. */
 gpunmf_status gpunmf_synchronize(gpunmf_handle h);
