@@ -58,6 +58,8 @@ struct SpParams {
     int a1_rows;
     float eps;
     int minus_one;
+    const float *W, *H;          // the FP32 factors, of n rows and rank r, for plain_wh
+    int n, r;
     const float *sum_partials;   // KL: [count][npad] partial sums of the other factor
     float *sum_out;              // [npad]
     int sum_count;
@@ -149,6 +151,12 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8])
                  : "memory");
 }
 
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float d;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+
 // s + c += x with the rounding error of s kept in c (Knuth's TwoSum), two sums at once: as good as sums
 // in FP64 at the FP32 pipe's rate (this GPU's FP64 pipe would take longer over V than reading it does)
 __device__ __forceinline__ void two_sum(float2 &s, float2 &c, float2 x) {
@@ -195,6 +203,14 @@ __device__ __noinline__ float2 sp_sums(uint32_t ta, int cols) {
         }
     }
     return make_float2(s.x + s.y, size.x + size.y);
+}
+
+// An element of W H by FP32 multiply-adds, where the sum of the parts' products is not finite: an infinity's later
+// parts are zero, so beside a zero or an infinity it has become NaN
+__device__ __noinline__ float plain_wh(const float *W, int n, const float *H, int r, int i, int u) {
+    float s = 0.f;
+    for (int a = 0; a < r && s == s; a++) s = fmaf(W[(long long)a * n + i], H[(long long)u * r + a], s);
+    return s;
 }
 
 // What the update kernel needs of the other factor, from the partials its own update left: this CTA's
@@ -499,8 +515,27 @@ __global__ void __launch_bounds__(NPC == 32 && MODE == kSpEuclid ? 768 : kSpThre
 #pragma unroll
             for (int c = 0; c < NC; c++) acc[c] = 0.f;
         }
+        // forms those of the columns h .. h + 7 of S again that are not finite, within the first `lim` columns
+        auto repair = [&](float (&s)[16], int h, int lim) {
+            bool odd = false;
+#pragma unroll
+            for (int c = 0; c < 8; c++) odd |= !(fabsf(s[h + c]) < kInf) && h + c < lim;
+            if (!__any_sync(0xffffffffu, odd)) return;
+            float again[8];
+#pragma unroll
+            for (int c = 0; c < 8; c++) again[c] = s[h + c];
+#pragma unroll 1
+            for (int c = 0; c < 8; c++) {
+                const int k = kk * kSpChunk + part * 16 + h + c, g = t * kTileM + row;
+                if (!(fabsf(again[c]) < kInf) && h + c < lim)
+                    again[c] = plain_wh(p.W, p.n, p.H, p.r, p.k_contig ? k : g, p.k_contig ? g : k);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 8; c++) s[h + c] = again[c];
+        };
         // the quality's terms of sixteen columns
-        auto sample = [&](const float (&v)[16], const float (&s)[16], int klim) {
+        auto sample = [&](const float (&v)[16], float (&s)[16], int klim) {
             if constexpr (MODE == kSpQuality || MODE == kSpKlQuality) {
                 uint32_t range = 0;
                 float2 l[8];
@@ -514,6 +549,8 @@ __global__ void __launch_bounds__(NPC == 32 && MODE == kSpEuclid ? 768 : kSpThre
                         two_sum(qs, qc, sub2(mul2(make_float2(v[2 * c], v[2 * c + 1]), l[c]), s2));
                     }
                 } else {  // the edge of V, or a sum that is zero, subnormal, infinite or NaN
+                    repair(s, 0, klim);
+                    repair(s, 8, klim);
 #pragma unroll
                     for (int c = 0; c < 16; c++)
                         if (c < klim)
@@ -643,10 +680,12 @@ __global__ void __launch_bounds__(NPC == 32 && MODE == kSpEuclid ? 768 : kSpThre
                         fine = fine && fabsf(q[c]) < 1e38f;
                     }
                     if (__any_sync(0xffffffffu, !fine || dmax > 8e37f || h + 8 > klim)) {
+                        const int lim = t * kTileM + row < p.a1_rows ? klim : 0;
+                        repair(s, h, lim);
 #pragma unroll
-                        for (int c = 0; c < 8; c += 2) {  // beyond K: 0 (not 0 / eps)
-                            const float x = h + c < klim ? v[h + c] / (s[h + c] + p.eps) - less : 0.f;
-                            const float y = h + c + 1 < klim ? v[h + c + 1] / (s[h + c + 1] + p.eps) - less : 0.f;
+                        for (int c = 0; c < 8; c += 2) {  // beyond V: 0 (not 0 / eps)
+                            const float x = h + c < lim ? v[h + c] / (s[h + c] + p.eps) - less : 0.f;
+                            const float y = h + c + 1 < lim ? v[h + c + 1] / (s[h + c + 1] + p.eps) - less : 0.f;
                             uint32_t a[3], b[3];
                             cut3(x, a[0], a[1], a[2]);
                             cut3(y, b[0], b[1], b[2]);
@@ -672,10 +711,12 @@ __global__ void __launch_bounds__(NPC == 32 && MODE == kSpEuclid ? 768 : kSpThre
                     for (int c = 0; c < 16; c++)
                         if (c >= klim) v[c] = s[c] = 0.f;
                 }
-                float most = 0.f;
+                float most = 0.f;  // (NaN if any is)
 #pragma unroll
-                for (int c = 0; c < 16; c++) most = fmaxf(most, fmaxf(fabsf(v[c]), fabsf(s[c])));
+                for (int c = 0; c < 16; c++) most = max_nan(most, max_nan(fabsf(v[c]), fabsf(s[c])));
                 if (__any_sync(0xffffffffu, most != 0.f && !(most >= 0x1p-40f && most <= 0x1p50f))) {
+                    repair(s, 0, klim);
+                    repair(s, 8, klim);
                     if (!(most >= 0x1p-40f && most <= 0x1p50f)) {
 #pragma unroll
                         for (int c = 0; c < 16; c++) {
@@ -745,8 +786,11 @@ __global__ void __launch_bounds__(NPC == 32 && MODE == kSpEuclid ? 768 : kSpThre
             if (j + 1 == nblk) drain(j, true);
         }
         if constexpr (kSum) {
-            double a = ((double)qs.x + (double)qc.x) + ((double)qs.y + (double)qc.y);
-            double b = ((double)ws.x + (double)wc.x) + ((double)ws.y + (double)wc.y);
+            // (beside an infinite sum its second term is NaN)
+            auto total = [](float2 s, float2 c) {
+                return (double)s.x + (fabsf(s.x) < kInf ? (double)c.x : 0.0) + ((double)s.y + (fabsf(s.y) < kInf ? (double)c.y : 0.0));
+            };
+            double a = total(qs, qc), b = total(ws, wc);
             if (MODE == kSpResidual) {
                 a += far_a;
                 b += far_b;
@@ -1088,6 +1132,7 @@ static void sp_setup(gpunmf_job *j, SpGemm &g, int rows, int K, bool k_contig, c
     p.wait_limit = kWaitLimitCycles;
     p.eps = j->eps;
     p.minus_one = rule_is_additive(j->rule);
+    p.W = j->W; p.H = j->H; p.n = j->n; p.r = j->r;
     g.smem = 1024 + p.sf * p.nbox * kSpFBox + p.sv * kSpVBytes + kSpBarBytes;
     p.ctas = g.grid = (int)std::min<long long>(t->max_ctas, (long long)p.tiles * p.kchunks);
     if (!tb) return;
@@ -1194,6 +1239,7 @@ static cudaError_t sp_update(gpunmf_job *j, bool is_w, int update) {
         u.sum_partials = is_w ? t->SP_w : t->SP_h;
         u.r = j->r; u.cols = rows; u.npad = t->npad; u.eps = j->eps; u.update = update;
         u.additive = rule_is_additive(j->rule) ? 2 : 0;  // 2: the - 1 is in the numerator already
+        u.V = j->V; u.W = j->W; u.H = j->H; u.n = j->n; u.m = j->m;
         u.checks = is_w ? t->C_w : t->C_h; u.row_sums = is_w ? t->Z_w : t->Z_h;
         u.low = sp_low_sum(is_w ? j->m : j->n); u.s_low = sp_low(t->npad / 16);
         return launch_kl_update(u, t->npad, is_w, j->stream);

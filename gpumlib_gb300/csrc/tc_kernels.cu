@@ -1589,11 +1589,17 @@ struct UpdParams {
     int slot0, slots;         // batches (slot_ptr null): the tile's slots, numbered on
 };
 
-// A numerator of the FP32 products by plain FP32 fused multiply-adds, where the sum of the parts'
-// products is not finite: a part of an infinity or NaN has lost which of the two it was.
-__device__ __noinline__ float plain_sum(int is_w, const float *V, long long ldv, const float *F, int r, int K, int row, int a) {
+#define kInf __int_as_float(0x7F800000)
+
+// The numerator `sum` of the FP32 products, which is not finite, by plain FP32 fused multiply-adds: a part of an
+// infinity or NaN has lost which of the two it was.  (Not where X is NaN, which decides without it; and a NaN
+// ends the sum.  One thread forms all of it, so a job that holds a NaN must not come here in every iteration.)
+__device__ __noinline__ float plain_sum(float sum, const float *X, long long ldx, int is_w, const float *V, long long ldv, const float *F,
+                                        int r, int K, int row, int a) {
+    const float x = is_w ? X[(long long)a * ldx + row] : X[(long long)row * r + a];
+    if (x != x) return sum;
     float s = 0.f;
-    for (int k = 0; k < K; k++)
+    for (int k = 0; k < K && s == s; k++)
         s = is_w ? fmaf(V[(long long)k * ldv + row], F[(long long)k * r + a], s)
                  : fmaf(V[(long long)row * ldv + k], F[(long long)a * K + k], s);
     return s;
@@ -1603,7 +1609,7 @@ __device__ __noinline__ float plain_sum(int is_w, const float *V, long long ldv,
 // low together, over the sum of their sizes; without any, what is expected.  (No cut of the tensor cores
 // comes near 2^-18: a sum that is off by more, infinite or NaN says nothing.)
 __device__ __forceinline__ float low_fraction(float d, float size, float expected) {
-    return size == 0.f ? expected : fabsf(d) <= size * 0x1p-18f ? __fdividef(d, size) : 0.f;
+    return size == 0.f ? expected : fabsf(d) <= size * 0x1p-18f && size < 0x1p126f ? __fdividef(d, size) : 0.f;
 }
 
 // The slots' checks of ROWS rows, summed by NT threads: neighbours take neighbouring rows (so that a warp's loads are
@@ -1666,6 +1672,23 @@ __host__ __device__ constexpr int upd_rows(int rows, int rp) {
 }
 __host__ __device__ constexpr int upd_threads(int rp) { return rp > 64 && rp <= 128 ? 512 : 256; }
 
+// Shared-memory loads that are issued where they stand (volatile).  Left to the compiler, how many of the update kernel's
+// were in flight together hung on the code around them: an iteration of 361 x 2429, r = 49, took 31 us or 44.
+template <int N>
+__device__ __forceinline__ void lds_now(const float *src, float (&v)[N]) {
+    const uint32_t at = smem_u32(src);
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4)
+            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3]) : "r"(at + 4 * i));
+    } else if constexpr (N == 2) {
+        asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "r"(at));
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i++) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[i]) : "r"(at + 4 * i));
+    }
+}
+
 // A thread's columns of the rank: vectors of four (or two) 16 vectors apart, so that the 16 threads of a
 // row read neighbouring vectors
 __host__ __device__ constexpr int upd_vec(int ta) { return ta % 4 == 0 ? 4 : ta % 2 == 0 ? 2 : 1; }
@@ -1678,7 +1701,7 @@ template <int TA>
 __device__ __forceinline__ void upd_lds(const float *row, int g, float (&v)[TA]) {
     constexpr int V = upd_vec(TA);
 #pragma unroll
-    for (int i = 0; i < TA; i += V) lds_vec<V>(row + upd_col<TA>(g, i), *reinterpret_cast<float (*)[V]>(&v[i]));
+    for (int i = 0; i < TA; i += V) lds_now<V>(row + upd_col<TA>(g, i), *reinterpret_cast<float (*)[V]>(&v[i]));
 }
 
 // rows c0 .. c0 + ROWS - 1 of the factor, by NT threads; part: the index of their Gram partial (BF16 jobs:
@@ -1687,6 +1710,7 @@ __device__ __forceinline__ void upd_lds(const float *row, int g, float (&v)[TA])
 template <int RP, int ROWS, int NT>
 __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part, float *sm) {
     constexpr int TA = RP / 16, RT = ROWS * 16 / NT;
+    constexpr int NB = TA <= 4 ? 8 : 4, NG = TA <= 4 ? 8 : TA <= 6 ? 4 : 2;  // steps whose operands are loaded together
     constexpr int LDX = ROWS + 4, LDN = RP + 4;
     float *Gs = sm;               // [RP][RP], zero outside r
     float *Xs = Gs + RP * RP;     // [RP][LDX]  the old X(a, row)
@@ -1742,9 +1766,16 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
     if (p.update) {
         // G (RP x RP; the rows of X beyond r are zero)
         constexpr int G4 = RP * RP / 4;
-#pragma unroll 4
-        for (int k = tid; k < G4; k += NT)
-            reinterpret_cast<float4 *>(Gs)[k] = __ldcg(reinterpret_cast<const float4 *>(p.G) + k);
+#pragma unroll 1
+        for (int k0 = tid; k0 < G4; k0 += 4 * NT) {
+            float4 g[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (k0 + q * NT < G4) g[q] = __ldcg(reinterpret_cast<const float4 *>(p.G) + k0 + q * NT);
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (k0 + q * NT < G4) reinterpret_cast<float4 *>(Gs)[k0 + q * NT] = g[q];
+        }
         // numerators: the tile's slots summed in their order, four slots' loads of a thread together.
         // (Rows of a slot beyond the last are in bounds, the tile has 128; they are never stored.)
         constexpr int N4 = ROWS * RP / 4;
@@ -1781,13 +1812,12 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
             }
             auto put = [&](int k, float4 v) {
                 const int c = k / (RP / 4), a = (k % (RP / 4)) * 4;
-                const float inf = __int_as_float(0x7F800000);
-                if (p.Xs && c < ncol && !(fabsf(v.x) < inf && fabsf(v.y) < inf && fabsf(v.z) < inf && fabsf(v.w) < inf)) {
-                    auto sum = [&](int aa) { return plain_sum(p.is_w, p.V, p.ldv, p.F, r, p.K, c0 + c, aa); };
-                    if (!(fabsf(v.x) < inf) && a < r) v.x = sum(a);
-                    if (!(fabsf(v.y) < inf) && a + 1 < r) v.y = sum(a + 1);
-                    if (!(fabsf(v.z) < inf) && a + 2 < r) v.z = sum(a + 2);
-                    if (!(fabsf(v.w) < inf) && a + 3 < r) v.w = sum(a + 3);
+                if (p.Xs && c < ncol && !(fabsf(v.x) < kInf && fabsf(v.y) < kInf && fabsf(v.z) < kInf && fabsf(v.w) < kInf)) {
+                    auto sum = [&](float s, int aa) { return plain_sum(s, p.X, p.ldx, p.is_w, p.V, p.ldv, p.F, r, p.K, c0 + c, aa); };
+                    if (!(fabsf(v.x) < kInf) && a < r) v.x = sum(v.x, a);
+                    if (!(fabsf(v.y) < kInf) && a + 1 < r) v.y = sum(v.y, a + 1);
+                    if (!(fabsf(v.z) < kInf) && a + 2 < r) v.z = sum(v.z, a + 2);
+                    if (!(fabsf(v.w) < kInf) && a + 3 < r) v.w = sum(v.w, a + 3);
                 }
                 *reinterpret_cast<float4 *>(Ns + c * LDN + a) = v;
             };
@@ -1802,15 +1832,20 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
         for (int i = 0; i < TA; i++)
 #pragma unroll
             for (int j = 0; j < RT; j++) den[i][j] = 0.f;
-#pragma unroll(TA <= 3 ? 16 : 4)
-        for (int b = 0; b < RP; b++) {
-            float xb[RT], g[TA];
-            lds_vec<RT>(Xs + b * LDX + gc * RT, xb);
-            upd_lds<TA>(Gs + b * RP, ga, g);
+#pragma unroll 1
+        for (int b = 0; b < RP; b += NB) {
+            float xb[NB][RT], g[NB][TA];
 #pragma unroll
-            for (int i = 0; i < TA; i++)
+            for (int q = 0; q < NB; q++) {
+                lds_now<RT>(Xs + (b + q) * LDX + gc * RT, xb[q]);
+                upd_lds<TA>(Gs + (b + q) * RP, ga, g[q]);
+            }
 #pragma unroll
-                for (int j = 0; j < RT; j++) den[i][j] = fmaf(g[i], xb[j], den[i][j]);
+            for (int q = 0; q < NB; q++)
+#pragma unroll
+                for (int i = 0; i < TA; i++)
+#pragma unroll
+                    for (int j = 0; j < RT; j++) den[i][j] = fmaf(g[q][i], xb[q][j], den[i][j]);
         }
         float low[RT];
 #pragma unroll
@@ -1899,15 +1934,20 @@ __device__ __forceinline__ void update_rows(const UpdParams &p, int c0, int part
                 for (int k = 0; k < TA; k++) acc[i][k] = 0.f;
 #pragma unroll 1
             for (int cb = c1; cb < c1 + step; cb += 16) {
-#pragma unroll(TA <= 4 ? 16 : 2)
-                for (int c = cb; c < cb + 16; c++) {
-                    float xa[TA], xb[TA];
-                    upd_lds<TA>(Ns + c * LDN, ga, xa);
-                    upd_lds<TA>(Ns + c * LDN, gb, xb);
+#pragma unroll(TA <= 4 ? 2 : 1)
+                for (int c = cb; c < cb + 16; c += NG) {
+                    float xa[NG][TA], xb[NG][TA];
 #pragma unroll
-                    for (int i = 0; i < TA; i++)
+                    for (int q = 0; q < NG; q++) {
+                        upd_lds<TA>(Ns + (c + q) * LDN, ga, xa[q]);
+                        upd_lds<TA>(Ns + (c + q) * LDN, gb, xb[q]);
+                    }
 #pragma unroll
-                        for (int k = 0; k < TA; k++) acc[i][k] = fmaf(xa[i], xb[k], acc[i][k]);
+                    for (int q = 0; q < NG; q++)
+#pragma unroll
+                        for (int i = 0; i < TA; i++)
+#pragma unroll
+                            for (int k = 0; k < TA; k++) acc[i][k] = fmaf(xa[q][i], xb[q][k], acc[i][k]);
                 }
             }
             if (H == 2 && p.Xs) {  // (G is read by no one any more: a barrier lies behind the denominators)
@@ -2657,7 +2697,26 @@ struct KlUpdParams {
     const float2 *checks;  // FP32 products: what the slots' rows are low by (UpdParams)
     float low, s_low;    // the fractions that a numerator (without a check) and S are expected to be low by
     float *row_sums;     // [cols] sums of X's rows (FP32 products)
+    const float *V, *W, *H;  // FP32 products: for plain_kl_terms
+    int n, m;
 };
+
+// The terms of a KL numerator of the FP32 products in which V is not finite, by plain FP32 operations: they alone say
+// whether the sum is infinite or NaN (an infinite quotient's parts have lost that; a finite one keeps it).  Of row `row`
+// of H' (or of W).
+__device__ __noinline__ float plain_kl_terms(int is_w, const float *V, const float *W, const float *H, int n, int m, int r, float eps,
+                                             int row, int a) {
+    float s = 0.f;
+    for (int k = 0; k < (is_w ? m : n) && s == s; k++) {
+        const int i = is_w ? row : k, u = is_w ? k : row;
+        const float v = V[(long long)u * n + i];
+        if (fabsf(v) < kInf) continue;
+        float wh = 0.f;
+        for (int b = 0; b < r && wh == wh; b++) wh = fmaf(W[(long long)b * n + i], H[(long long)u * r + b], wh);
+        s = fmaf(v / (wh + eps), is_w ? H[(long long)u * r + a] : W[(long long)a * n + i], s);
+    }
+    return s;
+}
 
 // COLS columns of H (rows of W) per CTA: 8 for the H-step (its m is the smaller side: more CTAs),
 // 16 for the W-step.  The old rows are staged in shared memory (W: read along its columns, H: along
@@ -2747,7 +2806,27 @@ __global__ void __launch_bounds__(kUpdThreads) tc_kl_update_kernel(KlUpdParams p
             }
         }
     }
-    __syncthreads();
+    bool odd = false;  // a numerator that is not finite
+#pragma unroll
+    for (int j = 0; j < XL; j++) odd |= !(fabsf(acc[j]) < kInf);
+    if (__syncthreads_or(odd && p.V)) {
+        // (not where X or the sum is NaN: they decide.  Of this factor the terms have their own row alone in
+        // them, which is written after the next barrier.)
+        float again[XL];
+#pragma unroll
+        for (int j = 0; j < XL; j++) again[j] = acc[j];
+#pragma unroll 1
+        for (int j = 0; j < XL; j++) {
+            const int k = tid + j * kUpdThreads, c = k / RP, a = k % RP;
+            if (c >= ncol || a >= r || fabsf(again[j]) < kInf) continue;
+            const float x = Xs[a * LDX + c];
+            if (x != x || sumS[a] != sumS[a]) continue;
+            const float s = plain_kl_terms(IS_W, p.V, p.W, p.H, p.n, p.m, r, p.eps, c0 + c, a);
+            if (!(fabsf(s) < kInf)) again[j] = s;
+        }
+#pragma unroll
+        for (int j = 0; j < XL; j++) acc[j] = again[j];
+    }
     if (checks) {
         if (tid < COLS) rowD[tid] = rc.fraction(row_checks, tid, p.low);
         __syncthreads();
@@ -3140,11 +3219,23 @@ static int update_smem_bytes(int rp, int rows) {
     return (rp * rp + rp * (rows + 4) + rows * (rp + 4)) * (int)sizeof(float);
 }
 
+// Shared memory that a CTA of an FP32 job's update asks for at least, so that no more of them share an SM than the grid
+// needs.  Their launch overlaps the product's end, when few SMs are free, and as many as fit pile up on
+// those: 361 x 2429, r = 49 (152 CTAs), took 44 us an iteration with four to an SM, 38 with three, 32 with two and 28 with
+// one; 8192 x 8192, r = 64 (512), 130 with four, 131 with two, 144 with one.  (Not for rank 16 and the KL updates, whose
+// CTAs do little: early ones are ready when the product ends.  1024 x 512, r = 16, 12.5 us an iteration and 13.7
+// spread, 3001 x 1777 additive KL, r = 40, 29 and 33.)
+constexpr int kSpreadMax = 228 * 1024 / 2 - 768;
+static int spread_smem(int grid) {
+    const int want = ceil_div(grid, num_sms());
+    return want <= 3 ? 228 * 1024 / (want + 1) - 768 : 0;
+}
+
 template <int RP>
 static cudaError_t set_update_smem_rp() {
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if constexpr (RP <= 64) {
-        return cudaFuncSetAttribute(tc_update_kernel<RP, 16>, attr, update_smem_bytes(RP, 16));
+        return cudaFuncSetAttribute(tc_update_kernel<RP, 16>, attr, std::max(kSpreadMax, update_smem_bytes(RP, 16)));
     } else {
         cudaError_t e = cudaFuncSetAttribute(tc_update_kernel<RP, 32>, attr, update_smem_bytes(RP, 32));
         if constexpr (RP <= 128)
@@ -3181,6 +3272,7 @@ static cudaError_t launch_update(const UpdParams &u, int rp, cudaStream_t s) {
     cfg.gridDim = dim3(ceil_div(u.cols, rows));
     cfg.blockDim = dim3(upd_threads(rp));
     cfg.dynamicSmemBytes = update_smem_bytes(rp, rows);
+    if (u.Xs && rp > 16 && rp <= 64) cfg.dynamicSmemBytes = std::max<size_t>(cfg.dynamicSmemBytes, spread_smem(cfg.gridDim.x));
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
