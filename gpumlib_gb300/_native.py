@@ -33,6 +33,9 @@ SIGNATURES = [
     ("gpunmf_set_quality_interval", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     ("gpunmf_set_wait_limit_cycles", ctypes.c_int, [ctypes.c_void_p, ctypes.c_longlong]),
     ("gpunmf_inject_missing_arrival", ctypes.c_int, [ctypes.c_void_p]),
+    ("gpunmf_inject_error_word", ctypes.c_int, [ctypes.c_void_p]),
+    ("gpunmf_batch_inject_error_word", ctypes.c_int, [ctypes.c_void_p]),
+    ("gpunmf_server_inject_error_word", ctypes.c_int, [ctypes.c_void_p]),
     ("gpunmf_set_grid_limit", ctypes.c_int, [ctypes.c_int]),
     ("gpunmf_quality_improvement", ctypes.c_int, [ctypes.c_void_p, c_float_p]),
     ("gpunmf_residual_fp64", ctypes.c_int, [ctypes.c_void_p, c_double_p]),

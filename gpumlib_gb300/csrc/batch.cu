@@ -478,7 +478,10 @@ struct gpunmf_batch {
     cudaGraphExec_t graph = nullptr;
     int graph_iters = -1;
     int grid = 0;
-    unsigned char *h_pinned = nullptr;  // page-locked room for the largest instance's W and H (gpunmf_batch_get)
+    // page-locked room: the error word, then the largest instance's W and H (gpunmf_batch_get); one call at a time
+    unsigned char *h_pinned = nullptr;
+    std::mutex mu;
+    bool ran = false, failed = false;  // launches whose error word has not been read; one of them gave up
     SpBatch *split = nullptr;  // the half-steps of all instances share their launches (split_batch.cuh)
 };
 
@@ -636,7 +639,7 @@ gpunmf_status gpunmf_batch_create(int count, const int *n, const int *m, const i
     }
     size_t largest = 0;
     for (const BatchInst &d : b->h_insts) largest = std::max(largest, sizeof(float) * (size_t)d.r * ((size_t)d.n + d.m));
-    if (cudaHostAlloc((void **)&b->h_pinned, largest, cudaHostAllocDefault) != cudaSuccess) {
+    if (cudaHostAlloc((void **)&b->h_pinned, 16 + largest, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();  // without it the copies go straight to the caller's memory
         b->h_pinned = nullptr;
     }
@@ -673,12 +676,37 @@ gpunmf_status gpunmf_batch_destroy(gpunmf_batch *b) {
     return GPUNMF_OK;
 }
 
+// Waits for the batch's stream and reports a wait of the kernels that ran out since the factors were set.  (The error
+// word's copy goes ahead of the wait, once after launches: on every read-back of 768 it cost 2 us each.)
+static gpunmf_status batch_wait(gpunmf_batch *b) {
+    int on_stack = 0;
+    int *word = b->h_pinned ? reinterpret_cast<int *>(b->h_pinned) : &on_stack;
+    const bool read = b->split && b->ran;
+    if (read) GPUNMF_CUDA_TRY(cudaMemcpyAsync(word, spb_error_word(b->split), sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+    GPUNMF_CUDA_TRY(cudaStreamSynchronize(b->stream));
+    if (read) {
+        b->ran = false;
+        if (*word != 0) b->failed = true;
+    }
+    if (b->failed) {
+        set_error("batch kernel gave up waiting");
+        return GPUNMF_ERR_TIMEOUT;
+    }
+    return GPUNMF_OK;
+}
+
 // Run `iters` iterations of every instance: the shared half-step launches, or one persistent launch,
 // captured in a CUDA graph (re-captured when iters changes) and replayed.  Returns without waiting.
 gpunmf_status gpunmf_batch_run(gpunmf_batch *b, int iters) {
     if (!b || iters < 0) return GPUNMF_ERR_INVALID;
     if (iters == 0) return GPUNMF_OK;
-    if (b->split) return spb_run(b->split, iters, b->stream);
+    if (b->split) {
+        {
+            std::lock_guard<std::mutex> lock(b->mu);
+            b->ran = true;
+        }
+        return spb_run(b->split, iters, b->stream);
+    }
     if (!b->graph || b->graph_iters != iters) {
         if (b->graph) {
             cudaGraphExecDestroy(b->graph);
@@ -705,8 +733,22 @@ gpunmf_status gpunmf_batch_run(gpunmf_batch *b, int iters) {
 
 gpunmf_status gpunmf_batch_synchronize(gpunmf_batch *b) {
     if (!b) return GPUNMF_ERR_INVALID;
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(b->stream));
-    return b->split ? spb_check(b->split, b->stream) : GPUNMF_OK;
+    std::lock_guard<std::mutex> lock(b->mu);
+    return batch_wait(b);
+}
+
+// Host-side fault injection: the error word of a batch whose instances share their launches stands as a kernel whose wait
+// ran out leaves it.
+gpunmf_status gpunmf_batch_inject_error_word(gpunmf_batch *b) {
+    if (!b) return GPUNMF_ERR_INVALID;
+    if (!b->split) {
+        set_error("this batch's kernel does not wait");
+        return GPUNMF_ERR_UNSUPPORTED;
+    }
+    std::lock_guard<std::mutex> lock(b->mu);
+    b->ran = true;
+    GPUNMF_CUDA_TRY(cudaMemsetAsync(spb_error_word(b->split), 1, 1, b->stream));
+    return GPUNMF_OK;
 }
 
 // Device time of `iters` iterations of the whole batch (one graph launch), in ms.
@@ -721,7 +763,10 @@ gpunmf_status gpunmf_batch_time(gpunmf_batch *b, int iters, float *ms) {
         cudaEventRecord(e0, b->stream);
         st = gpunmf_batch_run(b, iters);
         cudaEventRecord(e1, b->stream);
-        cudaEventSynchronize(e1);
+        if (st == GPUNMF_OK) {
+            std::lock_guard<std::mutex> lock(b->mu);
+            st = batch_wait(b);
+        }
         cudaEventElapsedTime(ms, e0, e1);
     }
     cudaEventDestroy(e0);
@@ -729,23 +774,33 @@ gpunmf_status gpunmf_batch_time(gpunmf_batch *b, int iters, float *ms) {
     return st;
 }
 
+static bool page_locked(const void *p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return false;
+}
+
 gpunmf_status gpunmf_batch_get(gpunmf_batch *b, int k, float *W, float *H) {
     if (!b || k < 0 || k >= b->count) return GPUNMF_ERR_INVALID;
     const BatchInst &d = b->h_insts[k];
     const size_t wb = sizeof(float) * (size_t)d.n * d.r, hb = sizeof(float) * (size_t)d.r * d.m;
+    std::lock_guard<std::mutex> lock(b->mu);
     // through page-locked memory: both copies are in flight at once and one wait ends them (to pageable
-    // memory each copy waits for itself: 33 us a call against 12)
+    // memory each copy waits for itself: 33 us a call against 12); the caller's own where it is that
     float *pw = W, *ph = H;
     if (b->h_pinned) {
-        pw = reinterpret_cast<float *>(b->h_pinned);
-        ph = pw + (size_t)d.n * d.r;
+        float *room = reinterpret_cast<float *>(b->h_pinned + 16);
+        if (W && !page_locked(W)) pw = room;
+        if (H && !page_locked(H)) ph = room + (size_t)d.n * d.r;
     }
     if (W) GPUNMF_CUDA_TRY(cudaMemcpyAsync(pw, b->W + d.w, wb, cudaMemcpyDeviceToHost, b->stream));
     if (H) GPUNMF_CUDA_TRY(cudaMemcpyAsync(ph, b->H + d.h, hb, cudaMemcpyDeviceToHost, b->stream));
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(b->stream));
+    const gpunmf_status st = batch_wait(b);
+    if (st != GPUNMF_OK && st != GPUNMF_ERR_TIMEOUT) return st;
     if (W && pw != W) memcpy(W, pw, wb);
     if (H && ph != H) memcpy(H, ph, hb);
-    return GPUNMF_OK;
+    return st;
 }
 
 // Relative residual of every instance (FP64 accumulation on the GPU).
@@ -754,8 +809,8 @@ gpunmf_status gpunmf_batch_residuals(gpunmf_batch *b, double *out) {
     batch_residual_kernel<<<b->count, 256, 0, b->stream>>>(b->d_insts, b->count, b->V, b->W, b->H, b->d_res);
     GPUNMF_CUDA_TRY(cudaGetLastError());
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(out, b->d_res, sizeof(double) * b->count, cudaMemcpyDeviceToHost, b->stream));
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(b->stream));
-    return GPUNMF_OK;
+    std::lock_guard<std::mutex> lock(b->mu);
+    return batch_wait(b);
 }
 
 // Tile configuration of instance k (see gpunmf_batch_configs); the rank class must match.
@@ -795,12 +850,13 @@ gpunmf_status gpunmf_batch_reset_factors(gpunmf_batch *b, const float *const *W,
         GPUNMF_CUDA_TRY(cudaMemcpyAsync(b->W + d.w, W[k], sizeof(float) * (size_t)d.n * d.r, cudaMemcpyHostToDevice, b->stream));
         GPUNMF_CUDA_TRY(cudaMemcpyAsync(b->H + d.h, H[k], sizeof(float) * (size_t)d.r * d.m, cudaMemcpyHostToDevice, b->stream));
     }
+    std::lock_guard<std::mutex> lock(b->mu);
     if (b->split) {
         gpunmf_status st = spb_reset(b->split, b->stream);
         if (st != GPUNMF_OK) return st;
     }
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(b->stream));
-    return GPUNMF_OK;
+    b->ran = b->failed = false;
+    return batch_wait(b);
 }
 
 }  // extern "C"

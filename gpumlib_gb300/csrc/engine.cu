@@ -724,6 +724,11 @@ gpunmf_status gpunmf_inject_missing_arrival(gpunmf_handle h) {
     return tc_inject_missing_arrival(h);
 }
 
+gpunmf_status gpunmf_inject_error_word(gpunmf_handle h) {
+    CHECK_HANDLE(h);
+    return job_inject_error(h);
+}
+
 gpunmf_status gpunmf_set_grid_limit(int ctas) {
     if (ctas < 0) {
         set_error("grid limit must be >= 0");
@@ -767,9 +772,9 @@ gpunmf_status gpunmf_objective_kl_fp64(gpunmf_handle h, double *out) {
     GPUNMF_CUDA_TRY(kl_objective_ew(h->V, h->WH, cnt, h->red, s));
     GPUNMF_CUDA_TRY(finalize_partials(h->red, ctas, 1, 0, nullptr, h->d_scalar, s));
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(h->h_scalar(), h->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, s));
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(s));
-    *out = h->h_scalar()[0];
-    return GPUNMF_OK;
+    const gpunmf_status st = tc_check_sync(h);
+    if (st == GPUNMF_OK || st == GPUNMF_ERR_TIMEOUT) *out = h->h_scalar()[0];
+    return st;
 }
 
 gpunmf_status gpunmf_get_w(gpunmf_handle h, float *W) {
@@ -791,8 +796,7 @@ gpunmf_status gpunmf_get_wh(gpunmf_handle h, float *WH) {
     if (!WH) return GPUNMF_ERR_INVALID;
     TRY_STATUS(ensure_wh(h));
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(WH, h->WH, sizeof(float) * (size_t)h->n * h->m, cudaMemcpyDeviceToHost, h->stream));
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return GPUNMF_OK;
+    return tc_check_sync(h);
 }
 
 gpunmf_status gpunmf_device_factors(gpunmf_handle h, float **dW, float **dH) {

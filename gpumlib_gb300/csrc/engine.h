@@ -105,7 +105,11 @@ gpunmf_status tc_quality(gpunmf_job *j);
 // fused Euclidean and KL jobs: the next H-step launch samples the quality itself (it also records the
 // job's quality event); false where it cannot
 bool tc_quality_fold(gpunmf_job *j);
-gpunmf_status tc_check_sync(gpunmf_job *j);  // waits for the job's stream and reads the kernels' error words
+// the kernels' error words into h_errors(), in stream order (not 0: a wait ran out); and what they say, once they are there
+gpunmf_status job_copy_errors(gpunmf_job *j);
+gpunmf_status job_errors(gpunmf_job *j);
+gpunmf_status tc_check_sync(gpunmf_job *j);  // copies them, waits for the job's stream and reads them
+gpunmf_status job_inject_error(gpunmf_job *j);  // sets an error word, as a kernel that gave up does
 void tc_set_wait_limit(gpunmf_job *j, long long cycles);  // <= 0: the default (about 2 s)
 gpunmf_status tc_inject_missing_arrival(gpunmf_job *j);
 void tc_set_grid_limit(int ctas);         // CTAs per launch of jobs created later (0: one per SM)
@@ -137,7 +141,7 @@ bool spb_better(const std::vector<SpbShape> &shapes);
 gpunmf_status spb_create(const std::vector<SpbShape> &shapes, float eps, cudaStream_t s, SpBatch **out);
 gpunmf_status spb_reset(SpBatch *b, cudaStream_t s);
 gpunmf_status spb_run(SpBatch *b, int iters, cudaStream_t s);
-gpunmf_status spb_check(SpBatch *b, cudaStream_t s);
+int *spb_error_word(SpBatch *b);  // device: not 0 once a wait of the kernels ran out
 void spb_destroy(SpBatch *b);
 // the job's relative residual, enqueued on its stream, into *d_out
 gpunmf_status job_residual(gpunmf_job *j, double *d_out);

@@ -119,6 +119,7 @@ constexpr int kServeMaxJobCtas = 24;
 struct gpunmf_server {
     int device = 0;
     std::atomic<int> blocks_per_cta{kServeBlocksPerCta}, max_job_ctas{kServeMaxJobCtas};
+    std::atomic<bool> inject{false};
     int slots = 0, precision = 0, check_every = 10, max_iters = 500;
     size_t budget = 0, in_use = 0;
     double tol = 1e-3;
@@ -153,7 +154,7 @@ static gpunmf_status chunk_body(gpunmf_server *S, SJob *q, int chunk) {
     st = job_residual(j, S->d_res + q->slot);
     if (st != GPUNMF_OK) return st;
     GPUNMF_CUDA_TRY(cudaMemcpyAsync(S->h_res + q->slot, S->d_res + q->slot, sizeof(double), cudaMemcpyDeviceToHost, s));
-    return GPUNMF_OK;
+    return job_copy_errors(j);
 }
 
 // Capture a full chunk into a CUDA graph, so that each later chunk is one graph launch
@@ -208,6 +209,7 @@ static gpunmf_status start_job(gpunmf_server *S, SJob *q) {
     st = generate_job_data(q->job, q->seed, S->sigma);
     if (st == GPUNMF_OK) st = job_prepare(q->job);
     if (st == GPUNMF_OK) job_residual_ready(q->job);
+    if (st == GPUNMF_OK && S->inject.exchange(false)) st = job_inject_error(q->job);
     if (st == GPUNMF_OK && S->max_iters >= S->check_every) st = capture_chunk(S, q);
     if (st == GPUNMF_OK) st = enqueue_chunk(S, q);
     return st;
@@ -294,6 +296,11 @@ static void worker_loop(gpunmf_server *S) {
                 continue;
             }
             q->res.residual = S->h_res[sl];
+            const gpunmf_status ran = job_errors(q->job);
+            if (ran != GPUNMF_OK) {  // a kernel of the chunk gave up waiting
+                finish_job(S, q, ran);
+                continue;
+            }
             if (q->res.residual <= S->tol || q->res.iters >= S->max_iters) {
                 finish_job(S, q, GPUNMF_OK);
             } else {
@@ -370,6 +377,12 @@ gpunmf_status gpunmf_server_set_grid_policy(gpunmf_server *S, int blocks_per_cta
     }
     S->blocks_per_cta.store(blocks_per_cta);
     S->max_job_ctas.store(max_job_ctas > 0 ? max_job_ctas : kServeMaxJobCtas);
+    return GPUNMF_OK;
+}
+
+gpunmf_status gpunmf_server_inject_error_word(gpunmf_server *S) {
+    if (!S) return GPUNMF_ERR_INVALID;
+    S->inject.store(true);
     return GPUNMF_OK;
 }
 

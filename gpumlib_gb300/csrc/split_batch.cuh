@@ -580,8 +580,9 @@ static cudaError_t spb_update(SpBatch *b, bool is_w, int update, cudaStream_t s)
     return spb_launch(spb_update_kernel, is_w ? b->blocks_w : b->blocks_h, kSpbUpdThreads, update_smem_bytes(kSpbNP, kSpbRows), s, u);
 }
 
-// After the factors have been written: their parts and the Gram partials of W.
+// After the factors have been written: their parts and the Gram partials of W.  (An error goes with the old ones.)
 gpunmf_status spb_reset(SpBatch *b, cudaStream_t s) {
+    GPUNMF_CUDA_TRY(cudaMemsetAsync(b->err, 0, sizeof(int), s));
     for (int i0 = 0; i0 < b->count; i0 += 65535) {
         spb_cut_kernel<<<dim3(4, std::min(65535, b->count - i0), 2), 256, 0, s>>>(b->insts + i0);
         GPUNMF_CUDA_TRY(cudaGetLastError());
@@ -600,17 +601,7 @@ gpunmf_status spb_run(SpBatch *b, int iters, cudaStream_t s) {
     return GPUNMF_OK;
 }
 
-// GPUNMF_ERR_TIMEOUT if a wait of the kernels ran out (after a synchronisation with s)
-gpunmf_status spb_check(SpBatch *b, cudaStream_t s) {
-    int e = 0;
-    GPUNMF_CUDA_TRY(cudaMemcpyAsync(&e, b->err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(s));
-    if (e != 0) {
-        set_error("batch kernel gave up waiting (error bits 0x%x)", e);
-        return GPUNMF_ERR_TIMEOUT;
-    }
-    return GPUNMF_OK;
-}
+int *spb_error_word(SpBatch *b) { return b->err; }
 
 void spb_destroy(SpBatch *b) {
     if (!b) return;

@@ -4026,17 +4026,37 @@ gpunmf_status tc_iterate(gpunmf_job *j, bool updateW) {
 // The kernels' error words, copied to the pinned block in the job's stream order (its memory may be
 // stream-ordered), ahead of the synchronisation the caller makes anyway: read by copies to the
 // stack and a synchronisation of their own they cost GetW and GetH 5 us each, a residual 18.
-gpunmf_status tc_check_sync(gpunmf_job *j) {
+gpunmf_status job_copy_errors(gpunmf_job *j) {
     const int *words[2] = {j->tc ? j->tc->err : nullptr, j->sp ? j->sp->err : nullptr};
-    int *e = j->h_errors();
-    e[0] = e[1] = 0;
     for (int k = 0; k < 2; k++)
-        if (words[k]) GPUNMF_CUDA_TRY(cudaMemcpyAsync(&e[k], words[k], sizeof(int), cudaMemcpyDeviceToHost, j->stream));
-    GPUNMF_CUDA_TRY(cudaStreamSynchronize(j->stream));
-    if (e[0] | e[1]) {
-        set_error("tensor-core kernel gave up waiting (error bits 0x%x)", e[0] | e[1]);
+        if (words[k])
+            GPUNMF_CUDA_TRY(cudaMemcpyAsync(&j->h_errors()[k], words[k], sizeof(int), cudaMemcpyDeviceToHost, j->stream));
+    return GPUNMF_OK;
+}
+
+gpunmf_status job_errors(gpunmf_job *j) {
+    const int e = (j->tc ? j->h_errors()[0] : 0) | (j->sp ? j->h_errors()[1] : 0);
+    if (e != 0) {
+        set_error("tensor-core kernel gave up waiting (error bits 0x%x)", e);
         return GPUNMF_ERR_TIMEOUT;
     }
+    return GPUNMF_OK;
+}
+
+gpunmf_status tc_check_sync(gpunmf_job *j) {
+    gpunmf_status st = job_copy_errors(j);
+    if (st != GPUNMF_OK) return st;
+    GPUNMF_CUDA_TRY(cudaStreamSynchronize(j->stream));
+    return job_errors(j);
+}
+
+gpunmf_status job_inject_error(gpunmf_job *j) {
+    int *word = j->tc ? j->tc->err : j->sp ? j->sp->err : nullptr;
+    if (!word) {
+        set_error("this job's kernels do not wait");
+        return GPUNMF_ERR_UNSUPPORTED;
+    }
+    GPUNMF_CUDA_TRY(cudaMemsetAsync(word, 1, 1, j->stream));
     return GPUNMF_OK;
 }
 

@@ -135,12 +135,15 @@ gpunmf_status gpunmf_set_quality_interval(gpunmf_handle h, int interval);
 
 /*
  * Bounded device waits (no counterpart in the reference, whose kernels never
- * wait on one another).  The BF16 kernels' CTAs wait on one another (tile
- * arrivals, grid-wide sums); every such wait gives up after a limit of SM
- * clock cycles, sets the job's error word, and the next call that reads it
- * (synchronize, get, residual) returns GPUNMF_ERR_TIMEOUT; the job must then be
- * destroyed.  Default limit: 4e9 cycles (about 2 s at 2 GHz); cycles <= 0
- * restores it.  Applies to the job's later launches.  BF16 jobs only.
+ * wait).  The tensor-core kernels wait: inside a CTA for copies and products,
+ * and the BF16 ones' CTAs on one another (tile arrivals, grid-wide sums).
+ * Every such wait gives up after a limit of SM clock cycles, sets the job's
+ * error word, and the next call that reads it (synchronize, get, residual,
+ * objective, time) returns GPUNMF_ERR_TIMEOUT; the job must then be destroyed.
+ * FP32 jobs up to rank 128 and batches report theirs in the same way, a batch
+ * until its factors are reset; a served job ends with that status.  Default
+ * limit: 4e9 cycles (about 2 s at 2 GHz); cycles <= 0 restores it.  This call
+ * changes the limit of a BF16 job's later launches (FP32 jobs keep the default).
  */
 gpunmf_status gpunmf_set_wait_limit_cycles(gpunmf_handle h, long long cycles);
 
@@ -152,6 +155,15 @@ gpunmf_status gpunmf_set_wait_limit_cycles(gpunmf_handle h, long long cycles);
  * GPUNMF_ERR_UNSUPPORTED for jobs without a fused update.
  */
 gpunmf_status gpunmf_inject_missing_arrival(gpunmf_handle h);
+
+/*
+ * Host-side fault injection: the job's error word stands as a kernel whose wait
+ * ran out leaves it, so that its next reading call returns GPUNMF_ERR_TIMEOUT.
+ * GPUNMF_ERR_UNSUPPORTED for jobs whose kernels do not wait (FP32 above rank
+ * 128).  gpunmf_batch_inject_error_word and gpunmf_server_inject_error_word (of
+ * the next job admitted) do the same.
+ */
+gpunmf_status gpunmf_inject_error_word(gpunmf_handle h);
 
 /*
  * CTAs per launch of the tensor-core kernels of jobs created after this call
@@ -264,6 +276,7 @@ gpunmf_status gpunmf_batch_synchronize(gpunmf_batch *b);
 gpunmf_status gpunmf_batch_time(gpunmf_batch *b, int iters, float *ms);
 /* Copy instance k's W (n x r) and/or H (r x m) to host buffers (NULL to skip). */
 gpunmf_status gpunmf_batch_get(gpunmf_batch *b, int k, float *W, float *H);
+gpunmf_status gpunmf_batch_inject_error_word(gpunmf_batch *b);
 /* Relative Frobenius residual of every instance (count doubles), FP64 on the GPU. */
 gpunmf_status gpunmf_batch_residuals(gpunmf_batch *b, double *out);
 /* Tile configurations of the persistent launch (a batch whose instances share their launches ignores
@@ -345,6 +358,7 @@ gpunmf_status gpunmf_server_submit(gpunmf_server *s, long long id, int rule, int
  * (as a job created alone does); max_job_ctas 0: the default cap.  Applies to jobs admitted after
  * the call.  Defaults: 1 block per CTA, at most 24 CTAs. */
 gpunmf_status gpunmf_server_set_grid_policy(gpunmf_server *s, int blocks_per_cta, int max_job_ctas);
+gpunmf_status gpunmf_server_inject_error_word(gpunmf_server *s);
 /* Move up to `cap` finished results into out[]; returns their number. */
 int gpunmf_server_poll(gpunmf_server *s, gpunmf_server_result *out, int cap);
 gpunmf_status gpunmf_server_fetch(gpunmf_server *s, long long id, gpunmf_server_result *res, float *W, float *H);
