@@ -65,6 +65,8 @@ SIGNATURES = [
     ("gpunmf_batch_time", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, c_float_p]),
     ("gpunmf_batch_get", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]),
     ("gpunmf_batch_residuals", ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
+    ("gpunmf_batch_shares_launches", ctypes.c_int, [ctypes.c_void_p]),
+    ("gpunmf_batch_share_launches", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     ("gpunmf_batch_configs", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     ("gpunmf_batch_set_config", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int]),
     ("gpunmf_batch_commit", ctypes.c_int, [ctypes.c_void_p]),

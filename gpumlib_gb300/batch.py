@@ -3,7 +3,7 @@
 ``Batch`` holds thousands of uneven Euclidean instances on the device and runs all of them at once: every
 half-step's launches shared by all instances (gpumlib_gb300/csrc/split_batch.cuh), or, where that is
 faster, one persistent, graph-captured launch with one CTA per instance
-(gpumlib_gb300/csrc/batch.cu).  ``autotune`` (of use for the latter) times every tile configuration
+(gpumlib_gb300/csrc/batch.cu).  ``autotune`` times, for the latter, every tile configuration
 of the matching rank class on a sample of each (rank class, size) bucket and
 assigns the fastest to every instance of that bucket.
 """
@@ -90,6 +90,14 @@ class Batch:
         _native.check(self._lib.gpunmf_batch_residuals(self._h, out.ctypes.data_as(_P)))
         return out
 
+    @property
+    def shares_launches(self):
+        """Whether the instances share their launches (else: one persistent launch, with tile configurations)."""
+        return bool(self._lib.gpunmf_batch_shares_launches(self._h))
+
+    def share_launches(self, on):
+        _native.check(self._lib.gpunmf_batch_share_launches(self._h, int(on)))
+
     def set_config(self, k, cfg):
         _native.check(self._lib.gpunmf_batch_set_config(self._h, int(k), int(cfg)))
         self.cfg[k] = cfg
@@ -124,7 +132,8 @@ class Batch:
 def autotune(batch, instances, sample=304, iters=3, seed=0):
     """Pick a tile configuration per (rank class, size class) bucket.
 
-    For each bucket, up to `sample` of its instances form a trial batch that
+    A batch whose instances share their launches has no use for one: each bucket gets the first of its rank
+    class, untimed.  Else, for each bucket, up to `sample` of its instances form a trial batch that
     is timed (device time, CUDA events) for `iters` iterations under every
     configuration of the bucket's rank class; the fastest is assigned to all
     of the bucket's instances in `batch`.  Returns {bucket: (cfg, {cfg: ms})}.
@@ -137,8 +146,14 @@ def autotune(batch, instances, sample=304, iters=3, seed=0):
     table = {}
     for key, members in sorted(buckets.items()):
         cands = [c for c, rc in enumerate(ranks) if rc == key[0]]
+        if batch.shares_launches:
+            table[key] = (cands[0], {})
+            for k in members:
+                batch.set_config(k, cands[0])
+            continue
         pick = members if len(members) <= sample else list(rng.choice(members, size=sample, replace=False))
         with Batch([instances[k] for k in pick]) as trial:
+            trial.share_launches(False)  # a smaller batch may be routed otherwise than the whole one
             timings = {}
             for c in cands:
                 for j in range(trial.count):

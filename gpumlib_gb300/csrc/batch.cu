@@ -483,6 +483,7 @@ struct gpunmf_batch {
     std::mutex mu;
     bool ran = false, failed = false;  // launches whose error word has not been read; one of them gave up
     SpBatch *split = nullptr;  // the half-steps of all instances share their launches (split_batch.cuh)
+    bool shared = false;       // and that is how it runs (never without split)
 };
 
 static int rank_class(int r) { return r <= 4 ? 4 : r <= 8 ? 8 : r <= 16 ? 16 : r <= 32 ? 32 : 0; }
@@ -657,8 +658,10 @@ gpunmf_status gpunmf_batch_create(int count, const int *n, const int *m, const i
         }
         if (spb_better(shapes)) {
             st = spb_create(shapes, eps, b->stream, &b->split);
-            if (st == GPUNMF_OK) st = spb_reset(b->split, b->stream);
-            else if (st == GPUNMF_ERR_NOMEM) st = GPUNMF_OK;  // the one-CTA kernel needs no more memory
+            if (st == GPUNMF_OK) {
+                st = spb_reset(b->split, b->stream);
+                b->shared = true;
+            } else if (st == GPUNMF_ERR_NOMEM) st = GPUNMF_OK;  // the one-CTA kernel needs no more memory
         }
     }
     if (st != GPUNMF_OK) {
@@ -700,7 +703,7 @@ static gpunmf_status batch_wait(gpunmf_batch *b) {
 gpunmf_status gpunmf_batch_run(gpunmf_batch *b, int iters) {
     if (!b || iters < 0) return GPUNMF_ERR_INVALID;
     if (iters == 0) return GPUNMF_OK;
-    if (b->split) {
+    if (b->shared) {
         {
             std::lock_guard<std::mutex> lock(b->mu);
             b->ran = true;
@@ -833,6 +836,26 @@ gpunmf_status gpunmf_batch_set_config(gpunmf_batch *b, int k, int cfg) {
 gpunmf_status gpunmf_batch_commit(gpunmf_batch *b) {
     if (!b) return GPUNMF_ERR_INVALID;
     return batch_upload_order(b);
+}
+
+// Whether the instances share their launches; and which of the two ways to run (GPUNMF_ERR_UNSUPPORTED for the shared
+// launches where the batch has none).  The factors stay as they are.
+int gpunmf_batch_shares_launches(const gpunmf_batch *b) { return b && b->shared; }
+
+gpunmf_status gpunmf_batch_share_launches(gpunmf_batch *b, int on) {
+    if (!b) return GPUNMF_ERR_INVALID;
+    if (on && !b->split) {
+        set_error("this batch has no shared launches");
+        return GPUNMF_ERR_UNSUPPORTED;
+    }
+    if (on && !b->shared) {  // (the other kernel keeps no parts of the factors)
+        std::lock_guard<std::mutex> lock(b->mu);
+        gpunmf_status st = batch_wait(b);
+        if (st == GPUNMF_OK) st = spb_reset(b->split, b->stream);
+        if (st != GPUNMF_OK) return st;
+    }
+    b->shared = on != 0;
+    return GPUNMF_OK;
 }
 
 // Number of tile configurations and the rank class of each (ranks[c], c < count).

@@ -282,6 +282,10 @@ gpunmf_status gpunmf_batch_residuals(gpunmf_batch *b, double *out);
 /* Tile configurations of the persistent launch (a batch whose instances share their launches ignores
  * them): returns their number; ranks[c] = rank class (4, 8, 16, 32) of config c. */
 int gpunmf_batch_configs(int *ranks, int cap);
+/* Whether the batch's instances share their launches (chosen at creation by what is faster), and a way to run it by the
+ * one persistent launch instead (on = 0) or by the shared ones again (GPUNMF_ERR_UNSUPPORTED where it has none). */
+int gpunmf_batch_shares_launches(const gpunmf_batch *b);
+gpunmf_status gpunmf_batch_share_launches(gpunmf_batch *b, int on);
 /* Choose instance k's tile configuration (same rank class), then commit before running. */
 gpunmf_status gpunmf_batch_set_config(gpunmf_batch *b, int k, int cfg);
 gpunmf_status gpunmf_batch_commit(gpunmf_batch *b);
