@@ -1081,15 +1081,16 @@ static cudaError_t sp_set_smem(int optin) {
 }
 
 static cudaError_t sp_set_smem_once() {
-    static std::once_flag once;
-    static cudaError_t result = cudaSuccess;
-    std::call_once(once, [] {
+    static OncePerDevice<cudaError_t> once;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return once.run(dev, [] {
         const int optin = smem_optin();
-        result = sp_set_smem<32>(optin);
+        cudaError_t result = sp_set_smem<32>(optin);
         if (result == cudaSuccess) result = sp_set_smem<64>(optin);
         if (result == cudaSuccess) result = sp_set_smem<128>(optin);
+        return result;
     });
-    return result;
 }
 
 template <int MODE>

@@ -43,6 +43,7 @@
 #include "common.cuh"
 #include "engine.h"
 #include "kernels.h"
+#include "once_per_device.h"
 #include "tc_ptx.cuh"
 
 namespace gpunmf {
@@ -3195,12 +3196,12 @@ static size_t gemm_partial_bytes(int rows, int K, int npad) {
 }
 
 static cudaError_t set_gemm_smem_once() {
-    static std::once_flag once;
-    static cudaError_t result = cudaSuccess;
-    std::call_once(once, [] {
-        int dev = 0, optin = 0;
-        cudaGetDevice(&dev);
-        result = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    static OncePerDevice<cudaError_t> once;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return once.run(dev, [dev] {
+        int optin = 0;
+        cudaError_t result = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (result == cudaSuccess)
             result = cudaFuncSetAttribute(tc_gemm_sk_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (result == cudaSuccess)
@@ -3211,8 +3212,8 @@ static cudaError_t set_gemm_smem_once() {
             result = cudaFuncSetAttribute(tc_gemm_sk_kernel<32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (result == cudaSuccess)
             result = cudaFuncSetAttribute(tc_gemm_sk_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        return result;
     });
-    return result;
 }
 
 static int update_smem_bytes(int rp, int rows) {
@@ -3314,12 +3315,12 @@ static UpdParams update_params_w(gpunmf_job *j, int update) {
 constexpr int kKlMaxRank = 128;
 
 static cudaError_t set_kl_smem_once() {
-    static std::once_flag once;
-    static cudaError_t result = cudaSuccess;
-    std::call_once(once, [] {
-        int dev = 0, optin = 0;
-        cudaGetDevice(&dev);
-        result = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    static OncePerDevice<cudaError_t> once;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return once.run(dev, [dev] {
+        int optin = 0;
+        cudaError_t result = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
 #define KLATTR(NK)                                                                                     \
     if (result == cudaSuccess)                                                                         \
         result = cudaFuncSetAttribute(tc_kl_gemm_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin); \
@@ -3327,8 +3328,8 @@ static cudaError_t set_kl_smem_once() {
         result = cudaFuncSetAttribute(tc_kl_gemm_kernel<NK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         KLATTR(1) KLATTR(2) KLATTR(3) KLATTR(4) KLATTR(5) KLATTR(6) KLATTR(7) KLATTR(8)
 #undef KLATTR
+        return result;
     });
-    return result;
 }
 
 // The stream of the last launch per device of a grid whose CTAs wait on one another (see
@@ -3677,10 +3678,11 @@ static gpunmf_status setup_quality(gpunmf_job *j) {
     if (st == GPUNMF_OK) st = make_map_tiled(&t->tmQV, t->Vbt, (uint64_t)(t->npr / 128) * (t->mpr / 64));
     q.kb64 = t->mpr / 64;
     if (st != GPUNMF_OK) return st;
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(tc_quality_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
+    static OncePerDevice<cudaError_t> once;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const cudaError_t attr = once.run(dev, [] {
+        return cudaFuncSetAttribute(tc_quality_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
     });
     if (attr != cudaSuccess) {
         set_error("cudaFuncSetAttribute (quality): %s", cudaGetErrorString(attr));
