@@ -1,7 +1,8 @@
 // NMF job engine: the C ABI of include/gpunmf.h.
 //
 // A job owns device copies of V, W and H plus every workspace its rule
-// needs, all allocated at creation (nothing is allocated per iteration).
+// needs, allocated at creation (nothing is allocated per iteration), but for
+// W H, when GetWH first asks for it, and what a BF16 job's first residual needs.
 // One iteration follows GPUMLib's order exactly:
 //   Euclidean (src/algorithms/nmf/nmf_multiplicative_euclidian.cpp:29-67)
 //     quality(W,H); H <- H .* (W'V) ./ (W'W H + eps); [W <- W .* (V H') ./ (W H H' + eps)]
@@ -134,16 +135,19 @@ static gpunmf_status dalloc(gpunmf_job *j, T **p, size_t count) {
 // ------------------------------------------------------------------------
 struct Sizes {
     int s_h, s_w, s_g;  // split-K slices: H-step product, W-step product, Gram products
-    size_t p_h, p_w, p_g, d_h, d_w, wh, red;
+    size_t p_h, p_w, p_g, d_h, d_w, wh, gram, sums, red;
 };
 
-static Sizes compute_sizes(int rule, int n, int m, int r, int precision) {
+// split: an FP32 job's products on the tensor cores, which have their own workspaces (sp_footprint)
+static Sizes compute_sizes(int rule, int n, int m, int r, int precision, bool split) {
     Sizes z{};
-    if (precision == GPUNMF_FP32 && sp_supported(n, m, r)) {  // products on the tensor cores: no FP32 workspaces
+    if (split) {
         z.s_h = z.s_w = z.s_g = 1;
         z.red = std::max(2 * (size_t)wh_reduce_ctas(n, m), (size_t)quality_ew_ctas((long long)n * m));
         return z;
     }
+    z.gram = (size_t)r * r;
+    z.sums = (size_t)r;
     z.s_h = gemm_f32_splits(r, m, n);
     z.s_w = gemm_f32_splits(n, r, m);
     int sg1 = gemm_f32_splits(r, r, n), sg2 = gemm_f32_splits(r, r, m);
@@ -163,9 +167,9 @@ static Sizes compute_sizes(int rule, int n, int m, int r, int precision) {
 }
 
 size_t job_footprint(int rule, int n, int m, int r, int precision) {
-    Sizes z = compute_sizes(rule, n, m, r, precision);
+    Sizes z = compute_sizes(rule, n, m, r, precision, precision == GPUNMF_FP32 && sp_supported(n, m, r));
     size_t floats = (size_t)n * m + (size_t)n * r + (size_t)r * m + z.p_h + z.p_w + z.p_g + z.d_h + z.d_w +
-                    z.wh + (size_t)r * r + (size_t)r + 8;
+                    z.wh + z.gram + z.sums + 8;
     size_t bytes = floats * sizeof(float) + z.red * sizeof(double) + 64;
     if (precision == GPUNMF_BF16) bytes += tc_footprint(rule, n, m, r);
     if (sp_supported(n, m, r)) bytes += sp_footprint(rule, n, m, r, precision == GPUNMF_BF16);
@@ -243,27 +247,14 @@ static gpunmf_status job_alloc(int rule, int n, int m, int r, float eps, int pre
         int dev = 0;
         if (cudaGetDevice(&dev) == cudaSuccess) j->pool = library_pool(dev);
     }
-    Sizes z = compute_sizes(rule, n, m, r, precision);
-    j->s_h = z.s_h; j->s_w = z.s_w; j->s_g = z.s_g;
     gpunmf_status st = GPUNMF_OK;
 #define ALLOC(ptr, cnt) \
     if (st == GPUNMF_OK) st = dalloc(j, &(ptr), (cnt));
     ALLOC(j->V, (size_t)n * m);
     ALLOC(j->W, (size_t)n * r);
     ALLOC(j->H, (size_t)r * m);
-    ALLOC(j->P_h, z.p_h);
-    ALLOC(j->P_w, z.p_w);
-    ALLOC(j->P_g, z.p_g);
-    ALLOC(j->G, (size_t)r * r);
-    ALLOC(j->D_h, z.d_h);
-    ALLOC(j->D_w, z.d_w);
-    ALLOC(j->WH, z.wh);
-    ALLOC(j->sums, (size_t)r);
     ALLOC(j->d_quality, 4);
-    ALLOC(j->red, z.red);
     ALLOC(j->d_scalar, 4);
-#undef ALLOC
-    j->red_cap = z.red;
     if (st == GPUNMF_OK && pinned64) {
         j->h_pinned = pinned64;
         j->external_pinned = true;
@@ -284,8 +275,27 @@ static gpunmf_status job_alloc(int rule, int n, int m, int r, float eps, int pre
             st = GPUNMF_ERR_CUDA;
         }
     }
+    if (st == GPUNMF_OK && precision == GPUNMF_FP32 && sp_supported(n, m, r)) {
+        st = sp_create(j, false);
+        if (st == GPUNMF_ERR_NOMEM) {  // tall matrices' Gram partials, V again with padded columns: the CUDA cores want less
+            sp_destroy(j);
+            st = GPUNMF_OK;
+        }
+    }
+    const Sizes z = compute_sizes(rule, n, m, r, precision, j->sp != nullptr);
+    j->s_h = z.s_h; j->s_w = z.s_w; j->s_g = z.s_g;
+    ALLOC(j->P_h, z.p_h);
+    ALLOC(j->P_w, z.p_w);
+    ALLOC(j->P_g, z.p_g);
+    ALLOC(j->G, z.gram);
+    ALLOC(j->D_h, z.d_h);
+    ALLOC(j->D_w, z.d_w);
+    ALLOC(j->WH, z.wh);
+    ALLOC(j->sums, z.sums);
+    ALLOC(j->red, z.red);
+#undef ALLOC
+    j->red_cap = z.red;
     if (st == GPUNMF_OK && precision == GPUNMF_BF16) st = tc_create(j);
-    if (st == GPUNMF_OK && precision == GPUNMF_FP32 && sp_supported(n, m, r)) st = sp_create(j, false);
     if (st != GPUNMF_OK) {
         job_free(j);
         return st;
