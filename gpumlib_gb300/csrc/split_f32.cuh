@@ -1,6 +1,6 @@
 // FP32 products on the tensor cores (included by tc_kernels.cu): every FP32 operand is cut into three
-// BF16 parts whose sum is the operand exactly (each the nearest BF16 of what is left), and a product
-// is the six BF16 products of parts whose weights are at least 2^-16 of the first one's:
+// BF16 parts whose sum is the operand (exactly above 2^-110: below, the last parts fall under BF16's smallest
+// numbers; each part the nearest BF16 of what is left), and a product is the six BF16 products of parts whose weights are at least 2^-16 of the first one's:
 //   x y = x0 y0 + (x0 y1 + x1 y0) + (x1 y1 + x0 y2 + x2 y0) + terms of either sign below 2^-23 x y
 // The tensor cores add in FP32 but do not round to nearest, so no long sum is left to them: an
 // accumulator in TMEM holds 64 of K (the five small products first, then the four K16 steps of
@@ -909,8 +909,8 @@ static int sp_class(int npad) { return npad <= 32 ? 32 : npad <= 64 ? 64 : 128; 
 bool sp_supported(int n, int m, int r) { return r <= kSpMaxRank && n > 0 && m > 0; }
 
 // CTAs of a product: stream-K over all SMs, but where that would cut a tile into more pieces than
-// the update kernels' slot table holds (few tiles), a whole number of CTAs per tile, at most
-// kSlotW of them.
+// the update kernels read at once (few tiles; the KL update's slot table holds kSlotW), a whole number of CTAs
+// per tile, at most kSlotW of them.
 static int sp_grid(int tiles, int kchunks, int max_ctas) {
     const long long T = (long long)tiles * kchunks;
     if (max_ctas / tiles + 2 > kSlotW)

@@ -1516,7 +1516,7 @@ __global__ void convert_h_kernel(const float *__restrict__ H, int r, int m, __nv
     }
 }
 
-// x = x0 + x1 + x2 exactly, each part the nearest BF16 of what is left, in the top half of a word (the
+// x = x0 + x1 + x2 (exactly above 2^-110), each part the nearest BF16 of what is left, in the top half of a word (the
 // FP32 products on the tensor cores, split_f32.cuh).  An infinity or NaN is its first part alone; a
 // value that would round to infinity is cut by truncation.
 __device__ __forceinline__ void cut3(float x, uint32_t &p0, uint32_t &p1, uint32_t &p2) {
