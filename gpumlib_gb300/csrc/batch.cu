@@ -484,6 +484,7 @@ struct gpunmf_batch {
     bool ran = false, failed = false;  // launches whose error word has not been read; one of them gave up
     SpBatch *split = nullptr;  // the half-steps of all instances share their launches (split_batch.cuh)
     bool shared = false;       // and that is how it runs (never without split)
+    cudaGraphExec_t shared_graph = nullptr;  // kSharedGraphIters iterations of it
 };
 
 static int rank_class(int r) { return r <= 4 ? 4 : r <= 8 ? 8 : r <= 16 ? 16 : r <= 32 ? 32 : 0; }
@@ -529,6 +530,7 @@ static void order_largest_first(const std::vector<BatchInst> &in, std::vector<in
 static void batch_free(gpunmf_batch *b) {
     if (!b) return;
     if (b->graph) cudaGraphExecDestroy(b->graph);
+    if (b->shared_graph) cudaGraphExecDestroy(b->shared_graph);
     spb_destroy(b->split);
     if (b->h_pinned) cudaFreeHost(b->h_pinned);
     void *ptrs[] = {b->d_insts, b->d_order, b->d_next, b->V, b->W, b->H, b->d_res};
@@ -698,6 +700,26 @@ static gpunmf_status batch_wait(gpunmf_batch *b) {
     return GPUNMF_OK;
 }
 
+// The shared launches are four an iteration, and a stream takes about a thousand before the caller has to wait: long
+// runs go by graphs of kSharedGraphIters iterations.
+constexpr int kSharedGraphIters = 64;
+static gpunmf_status batch_run_shared(gpunmf_batch *b, int iters) {
+    if (iters > 2 * kSharedGraphIters) {
+        if (!b->shared_graph) {
+            cudaGraph_t g = nullptr;
+            GPUNMF_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+            gpunmf_status st = spb_run(b->split, kSharedGraphIters, b->stream);
+            cudaError_t e = cudaStreamEndCapture(b->stream, &g);
+            if (e == cudaSuccess && st == GPUNMF_OK) e = cudaGraphInstantiate(&b->shared_graph, g, 0);
+            if (g) cudaGraphDestroy(g);
+            if (st != GPUNMF_OK) return st;
+            GPUNMF_CUDA_TRY(e);
+        }
+        for (; iters >= kSharedGraphIters; iters -= kSharedGraphIters) GPUNMF_CUDA_TRY(cudaGraphLaunch(b->shared_graph, b->stream));
+    }
+    return spb_run(b->split, iters, b->stream);
+}
+
 // Run `iters` iterations of every instance: the shared half-step launches, or one persistent launch,
 // captured in a CUDA graph (re-captured when iters changes) and replayed.  Returns without waiting.
 gpunmf_status gpunmf_batch_run(gpunmf_batch *b, int iters) {
@@ -708,7 +730,7 @@ gpunmf_status gpunmf_batch_run(gpunmf_batch *b, int iters) {
             std::lock_guard<std::mutex> lock(b->mu);
             b->ran = true;
         }
-        return spb_run(b->split, iters, b->stream);
+        return batch_run_shared(b, iters);
     }
     if (!b->graph || b->graph_iters != iters) {
         if (b->graph) {
