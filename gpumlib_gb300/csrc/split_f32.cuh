@@ -930,8 +930,10 @@ static int sp_grid(int tiles, int kchunks, int max_ctas) {
 // After 100 iterations of 42 generated jobs (64 .. 2048 rows and columns, ranks 8 .. 64) the factors are 1.0e-6 off (rms;
 // largest 1.7e-6), as with FP32 multiply-adds (1.0e-6, 1.6e-6); with every second chunk scaled by 1 + 2^-23, so that sums
 // of few chunks got up to twice their share, 2.0e-6 and 4.5e-6.  With W spread over twenty-five powers of two, 0.4e-6
-// .. 4.9e-6 (multiply-adds 0.4e-6 .. 2.2e-6; the table alone 9e-6).  The price: 8192 x 8192 a product of 55.0 us
-// for 53.5 (r = 64), 75.5 for 74.5 (r = 128); an iteration of 1024 x 512, r = 16, 16.4 us for 14.2.
+// .. 4.9e-6 (multiply-adds 0.4e-6 .. 2.2e-6; the table alone 9e-6).  The price: 8192 x 8192 a product of 55.2 us
+// for 53.5 (r = 64), 75.6 for 74.6 (r = 128); an iteration of 1024 x 512, r = 16, 15.5 us for 14.5; a KL half-step of 361 x 472,
+// r = 49, 4.9 us for 4.3.  Checks in a CTA's last chunk and at every tile's start, behind the drain of the chunk before,
+// measured the same there and slower at rank 128 (80.5 us a product).
 constexpr float kSpLow[9] = {0.f, 0.70f, 0.82f, 0.95f, 1.10f, 1.57f, 1.78f, 2.06f, 2.34f};
 static float sp_low(int steps) { return kSpLow[steps] * 0x1p-24f; }
 // a numerator's fraction: its chunks of 64 (and a last one of fewer) weighted by their share of K

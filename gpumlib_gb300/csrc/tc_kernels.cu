@@ -3223,12 +3223,13 @@ static int update_smem_bytes(int rp, int rows) {
 // Shared memory that a CTA of an FP32 job's update asks for at least, so that no more of them share an SM than the grid
 // needs.  Their launch overlaps the product's end, when few SMs are free, and as many as fit pile up on
 // those: 361 x 2429, r = 49 (152 CTAs), took 44 us an iteration with four to an SM, 38 with three, 32 with two and 28 with
-// one; 8192 x 8192, r = 64 (512), 130 with four, 131 with two, 144 with one.  (Not for rank 16 and the KL updates, whose
-// CTAs do little: early ones are ready when the product ends.  1024 x 512, r = 16, 12.5 us an iteration and 13.7
-// spread, 3001 x 1777 additive KL, r = 40, 29 and 33.)
+// one; 8192 x 8192, r = 64 (512), 130 with four, 131 with two, 144 with one.  CTAs that do little are better early than
+// alone: at least two to an SM for rank 16 (1024 x 512: 15.5 us an iteration with two, 15.3 with one, 17.8 with five, after a
+// sample 12.4, 13.9 and 12.6; 3000 x 2000, r = 10: 25.2, 28.0 and 26.5), and no limit for the KL updates (3001 x 1777
+// additive, r = 40: 30 without, 32 with two).
 constexpr int kSpreadMax = 228 * 1024 / 2 - 768;
-static int spread_smem(int grid) {
-    const int want = ceil_div(grid, num_sms());
+static int spread_smem(int grid, int least) {
+    const int want = std::max(least, ceil_div(grid, num_sms()));
     return want <= 3 ? 228 * 1024 / (want + 1) - 768 : 0;
 }
 
@@ -3273,7 +3274,7 @@ static cudaError_t launch_update(const UpdParams &u, int rp, cudaStream_t s) {
     cfg.gridDim = dim3(ceil_div(u.cols, rows));
     cfg.blockDim = dim3(upd_threads(rp));
     cfg.dynamicSmemBytes = update_smem_bytes(rp, rows);
-    if (u.Xs && rp > 16 && rp <= 64) cfg.dynamicSmemBytes = std::max<size_t>(cfg.dynamicSmemBytes, spread_smem(cfg.gridDim.x));
+    if (u.Xs && rp <= 64) cfg.dynamicSmemBytes = std::max<size_t>(cfg.dynamicSmemBytes, spread_smem(cfg.gridDim.x, rp > 16 ? 1 : 2));
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
