@@ -166,8 +166,8 @@ gpunmf_status gpunmf_inject_missing_arrival(gpunmf_handle h);
 gpunmf_status gpunmf_inject_error_word(gpunmf_handle h);
 
 /*
- * CTAs per launch of the tensor-core kernels of jobs created after this call
- * (0 = one per SM, the default).  The fused kernels need their whole grid
+ * CTAs per launch of the tensor-core kernels of BF16 jobs created after this call
+ * (0 = one per SM, the default; FP32 jobs' CTAs do not wait on one another).  The fused kernels need their whole grid
  * resident at once; an application that keeps long-running kernels of its own
  * on some SMs (persistent kernels of another library, on other streams) caps
  * the grid below the SMs those leave free, so the fused grid never waits for
@@ -179,7 +179,8 @@ gpunmf_status gpunmf_set_grid_limit(int ctas);
 gpunmf_status gpunmf_quality_improvement(gpunmf_handle h, float *out);
 
 /* Relative Frobenius residual ||V - W H||_F / ||V||_F of the current factors,
- * WH in FP32 from the FP32 factors, squares accumulated in FP64 on the GPU. */
+ * WH to FP32 accuracy from the FP32 factors, squares and sums to FP64's (in two FP32 terms, or in FP64 where
+ * the squares leave FP32's range).  NaN where V holds one. */
 gpunmf_status gpunmf_residual_fp64(gpunmf_handle h, double *out);
 
 /*
